@@ -28,10 +28,11 @@ static __device__ __align__(256) float4 g_static_scratch[kStaticScratchPoints];
 
 std::mutex g_setup_mutex;
 float4* g_scratch_addr[kMaxDevices] = {};
+int g_num_sms[kMaxDevices] = {};
 
 // The array's device address on `device` (the host-side name is only a stand-in, never a device
-// address).  Looked up once per device with that device current.
-int scratch_address(int device, float4** out) {
+// address) and the device's SM count.  Looked up once per device with that device current.
+int scratch_address(int device, float4** out, int* num_sms) {
     if (device < 0 || device >= kMaxDevices) {
         set_error("device %d out of range for the static scratch table", device);
         return LPM_ERR_ARG;
@@ -41,9 +42,11 @@ int scratch_address(int device, float4** out) {
         void* p = nullptr;
         const cudaError_t e = cudaGetSymbolAddress(&p, g_static_scratch);
         if (e != cudaSuccess) return cuda_status(e, "cudaGetSymbolAddress (static scratch)");
+        LPM_CUDA_TRY(cudaDeviceGetAttribute(&g_num_sms[device], cudaDevAttrMultiProcessorCount, device));
         g_scratch_addr[device] = (float4*)p;
     }
     *out = g_scratch_addr[device];
+    *num_sms = g_num_sms[device];
     return LPM_OK;
 }
 
@@ -72,12 +75,14 @@ extern "C" int lpm_direct_sum_f32_noalloc(const lpm_kernel_desc* kernel, const d
     int device = 0;
     LPM_CUDA_TRY(cudaGetDevice(&device));
     float4* s32 = nullptr;
-    rc = scratch_address(device, &s32);
+    int num_sms = 0;
+    rc = scratch_address(device, &s32, &num_sms);
     if (rc) return rc;
     float4* t32 = s32 + n_src;
     // a context on the stack: launches only, no buffers, no profiling events
     lpm_ctx local;
     local.device = device;
+    local.num_sms = num_sms;
     local.stream = (cudaStream_t)cuda_stream;
     rc = pack_f32(&local, (const double4*)src, n_src, s32, kernel->kind == LPM_KERNEL_BIOT_SAVART_SPHERE);
     if (rc) return rc;

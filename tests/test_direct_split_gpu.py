@@ -1,0 +1,103 @@
+"""Direct sums at the sizes where their source splits change: thread groups, cluster parts, ragged tiles and targets.
+
+Tolerances.  FP64: each of the at most n_src terms and their sum round within 2^-53 of sum |terms|, and a close pair's
+denominator within 2^-53 / den, 2e-12 of the pair at the closest spacing here; against the largest component 1e-12 (as
+the other FP64 parity tests).  FP32: 5e-6 relative L2 (as the other FP32 tests).  Sums that differ only in the order of
+their FP64 additions: 1e-13.
+"""
+import numpy as np
+import pytest
+
+import lpmcxx_b200 as L
+import oracle
+from conftest import rel_l2, rel_linf
+from test_direct_sum_gpu import random_sphere
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [(2, 1), (63, 129), (64, 128), (127, 511), (512, 513), (513, 31), (1025, 1025), (2049, 4735), (5121, 7777),
+         (16385, 300), (300, 60001)]
+
+
+def _data(n_src, n_tgt, scalar):
+    rng = np.random.default_rng(n_src + 3 * n_tgt)
+    n = max(n_src, n_tgt)
+    pts = rng.uniform(-1.0, 1.0, (n, 3)) if scalar else random_sphere(n, n)
+    src = oracle.pack4(pts[:n_src], rng.uniform(-1, 1, n_src) / n_src)
+    return src, oracle.pack4(pts[:n_tgt])
+
+
+def _sum(ctx, kernel, prec, src, tgt, comps, coinc):
+    import torch
+
+    out = torch.full((comps, tgt.shape[0]), float("nan"), dtype=torch.float64, device="cuda")
+    ctx.direct_sum_dev(kernel, prec, torch.tensor(src, device="cuda"), torch.tensor(tgt, device="cuda"), out, coinc)
+    return out.cpu().numpy()
+
+
+@pytest.mark.parametrize("n_src,n_tgt", SIZES)
+@pytest.mark.parametrize("delta", [0.0, 0.03])
+def test_biot_savart_split(ctx, n_src, n_tgt, delta):
+    ctx.use_torch_stream()
+    src, tgt = _data(n_src, n_tgt, False)
+    kernel, coinc = L.biot_savart_kernel(1.0, delta), min(n_src, n_tgt)
+    ref = oracle.bs_direct(src, tgt, delta=delta)
+    got = _sum(ctx, kernel, L.LPM_PREC_F64, src, tgt, 3, coinc)
+    assert rel_linf(got, ref) < 1e-12
+    if not np.any(ref):
+        return
+    first = None
+    for targets in (2, 4, 8):
+        ctx.set_param("direct_targets", targets)
+        f32 = _sum(ctx, kernel, L.LPM_PREC_F32, src, tgt, 3, coinc)
+        ctx.set_param("direct_targets", 4)
+        assert rel_l2(f32, ref) < 5e-6
+        first = f32 if first is None else first
+        assert rel_linf(f32, first) < 1e-13
+
+
+@pytest.mark.parametrize("n_src,n_tgt", SIZES)
+def test_poisson_split(ctx, n_src, n_tgt):
+    ctx.use_torch_stream()
+    src, tgt = _data(n_src, n_tgt, True)
+    ref = oracle.poisson_direct(src, tgt)
+    got = _sum(ctx, L.poisson_kernel(), L.LPM_PREC_F64, src, tgt, 1, min(n_src, n_tgt))[0]
+    assert rel_linf(got, ref) < 1e-12
+    f32 = _sum(ctx, L.poisson_kernel(), L.LPM_PREC_F32, src, tgt, 1, min(n_src, n_tgt))[0]
+    if np.any(ref):
+        assert rel_l2(f32, ref) < 5e-6
+
+
+def test_reciprocals_to_the_last_bits(ctx):
+    """One pair per target (the other sources have strength 0): r (1 + e + e^2) and y (1 + e (1/2 + 3/8 e)) against
+    80-bit results.  Biot-Savart: three roundings of den (3 2^-53 / den), five more of the product and cross product."""
+    ctx.use_torch_stream()
+    n = 4001
+    t = np.linspace(0.06, np.pi, n)
+    tgt = oracle.pack4(np.stack([np.cos(t), np.sin(t), np.zeros(n)], axis=1))
+    src = oracle.pack4(np.tile([0.0, 0.0, 1.0], (300, 1)))
+    src[100] = (1.0, 0.0, 0.0, 1.0)
+    got = _sum(ctx, L.biot_savart_kernel(), L.LPM_PREC_F64, src, tgt, 3, 0)[2]
+    x = tgt.astype(np.longdouble)
+    den = 1 - x[:, 0]
+    ref = x[:, 1] / den / (4 * np.longdouble(np.pi))  # -(x cross y)_z / (4 pi den), y = (1, 0, 0)
+    assert np.max(np.abs(got / ref - 1) / (2.0 ** -53 * (8 + 3 / den))) < 1.0
+    phi = _sum(ctx, L.poisson_kernel(), L.LPM_PREC_F64, src, tgt, 1, 0)[0]
+    r = np.sqrt((x[:, 0] - 1) ** 2 + x[:, 1] ** 2)
+    assert np.max(np.abs(phi * (4 * np.longdouble(np.pi)) * r - 1)) < 8 * 2.0 ** -53
+
+
+def test_values_that_are_not_finite(ctx):
+    """A NaN coordinate spoils the components it enters and no others, as the reference's expression does."""
+    ctx.use_torch_stream()
+    src, tgt = _data(700, 300, False)
+    src[400, 0] = np.nan
+    got = _sum(ctx, L.biot_savart_kernel(), L.LPM_PREC_F64, src, tgt, 3, 0)
+    assert np.isfinite(got[0]).all() and np.isnan(got[1:]).all()
+    tgt2 = tgt.copy()
+    tgt2[7, :3] = np.nan
+    clean, _ = _data(700, 300, False)
+    got = _sum(ctx, L.biot_savart_kernel(), L.LPM_PREC_F64, clean, tgt2, 3, 0)
+    assert np.isnan(got[:, 7]).all() and np.isfinite(np.delete(got, 7, axis=1)).all()
+    phi = _sum(ctx, L.poisson_kernel(), L.LPM_PREC_F64, src, tgt, 1, 0)[0]
+    assert rel_linf(phi, oracle.poisson_direct(np.delete(src, 400, axis=0), tgt)) < 1e-12
