@@ -10,6 +10,10 @@
 // key ranges split level by level on the GPU: a node at level l with more than max_per_leaf points
 // splits into the non-empty ranges of its points' level-(l+1) digits.  Sorted order is the
 // reference's depth-first order, so leaves sorted by range start are its leaves in DFS order.
+//
+// The short dependent phases (the passes of a sort of up to 131,072 keys, the levels of the split, the leaf
+// numbering) each run as ONE launch of a single thread-block cluster, whose blocks meet at the hardware cluster
+// barrier (release / acquire, so the global memory they write is visible across it) instead of at launch boundaries.
 #include "octree.h"
 
 #include <algorithm>
@@ -103,6 +107,42 @@ __global__ void scan_apply_kernel(const int32_t* __restrict__ in, int32_t* __res
     }
 }
 
+// ---------------------------------------------------------------------------------- one cluster
+constexpr int kClBlocks = 8;  // portable cluster size
+constexpr int kClThreads = 1024;
+constexpr int kClWarps = kClBlocks * kClThreads / 32;
+
+// Every thread of the cluster's blocks; orders their memory accesses (release / acquire at cluster scope).
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;\n" ::: "memory");
+}
+// The int at `p` of this block's shared memory, read from the block of rank `rank`.
+__device__ __forceinline__ int32_t cluster_load(const int32_t* p, int rank) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(p);
+    int32_t v;
+    asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %1, %2;\n\tld.shared::cluster.s32 %0, [ra];\n\t}"
+                 : "=r"(v)
+                 : "r"(s), "r"(rank)
+                 : "memory");
+    return v;
+}
+
+// The block's total v over all blocks (*total) and over the blocks of lower rank (returned).  One cluster barrier
+// inside; `slot` (one int of shared memory) may be written again only after the next one.
+__device__ __forceinline__ int32_t cluster_excl(int32_t v, int32_t* slot, int rank, int32_t* total) {
+    if (threadIdx.x == 0) *slot = v;
+    cluster_barrier();
+    int32_t before = 0, all = 0;
+#pragma unroll
+    for (int r = 0; r < kClBlocks; ++r) {
+        const int32_t t = cluster_load(slot, r);
+        all += t;
+        before += r < rank ? t : 0;
+    }
+    *total = all;
+    return before;
+}
+
 // ---------------------------------------------------------------------------------- radix sort
 template <typename K>
 __global__ void __launch_bounds__(kSortThreads) radix_hist_kernel(const K* __restrict__ keys, int64_t n, int shift,
@@ -111,11 +151,15 @@ __global__ void __launch_bounds__(kSortThreads) radix_hist_kernel(const K* __res
     h[threadIdx.x] = 0;
     __syncthreads();
     const int64_t base = (int64_t)blockIdx.x * kSortTile;
-#pragma unroll 4
+    int d[kSortItems];
+#pragma unroll
     for (int k = 0; k < kSortItems; ++k) {
         const int64_t i = base + k * kSortThreads + threadIdx.x;
-        if (i < n) atomicAdd(&h[(int)((keys[i] >> shift) & 255)], 1);
+        d[k] = i < n ? (int)((keys[i] >> shift) & 255) : -1;
     }
+#pragma unroll
+    for (int k = 0; k < kSortItems; ++k)
+        if (d[k] >= 0) atomicAdd(&h[d[k]], 1);
     __syncthreads();
     counts[(int64_t)threadIdx.x * nblocks + blockIdx.x] = h[threadIdx.x];
 }
@@ -177,6 +221,188 @@ __global__ void __launch_bounds__(kSortThreads) radix_scatter_kernel(const K* __
     }
 }
 
+// ---- packed keys: the sorted bits in the upper 32, the item's index in the lower 32 (morton_keys_kernel writes them so
+// where no lower key bit is sorted or read), so that a pass moves 8 bytes an item instead of 12 and reads them once:
+// a thread keeps its keys and their ranks in registers, the block orders its tile in shared memory and writes it out in
+// runs of equal digits.
+
+// Ranks of a warp's keys (key[j] at position 32 j + lane of its segment of `per` items, `n` of them valid) among its keys
+// of the same digit, in segment order, two 16-bit ranks a word; the warp's digit counts are left in wh (zeroed before).
+template <int ITEMS>
+__device__ __forceinline__ void warp_ranks(const uint64_t (&key)[ITEMS], int per, int n, int shift, int32_t* wh,
+                                           uint32_t (&rank2)[(ITEMS + 1) / 2]) {
+    const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+        if (j % 2 == 0) rank2[j / 2] = 0;
+        if (32 * j >= per) continue;  // warp-uniform
+        const bool valid = 32 * j + lane < n;
+        const int d = valid ? (int)((key[j] >> shift) & 255) : 256;
+        const unsigned peers = __match_any_sync(0xffffffffu, d);
+        const int32_t before = valid ? wh[d] : 0;
+        __syncwarp();
+        if (valid && (peers & lt) == 0) wh[d] = before + __popc(peers);
+        __syncwarp();
+        rank2[j / 2] |= (uint32_t)(before + __popc(peers & lt)) << (16 * (j % 2));
+    }
+}
+
+// The whole LSD sort of n <= ITEMS x 8192 packed keys by one cluster: every pass ranks, exchanges the blocks' digit
+// counts through distributed shared memory and writes, two cluster barriers a pass instead of three to five launches.
+// The last pass writes perm too.  Bound by the latency of its phases (one global round trip, 256-digit scans, two
+// barriers); 8 SMs suffice up to 131,072 keys, above that the many-block passes below are faster.
+template <int ITEMS>
+struct ClusterSortShape {
+    static constexpr int kWarps = kClThreads / 32;
+    static constexpr size_t kSmem = sizeof(uint64_t) * ITEMS * kClThreads + sizeof(int32_t) * (kWarps * 256 + 3 * 256);
+};
+template <int ITEMS>
+__global__ void __cluster_dims__(kClBlocks, 1, 1) __launch_bounds__(kClThreads)
+    cluster_sort_kernel(uint64_t* __restrict__ keys, uint64_t* __restrict__ tk, int32_t* __restrict__ perm, int n,
+                        int bit_lo) {
+    constexpr int kW = kClThreads / 32;
+    extern __shared__ __align__(16) uint64_t tile[];
+    int32_t* const wh = (int32_t*)(tile + ITEMS * kClThreads);  // [warp][digit]
+    int32_t* const tot = wh + kW * 256;
+    int32_t* const start = tot + 256;  // the block's first position of each digit
+    int32_t* const out = start + 256;  // global position of a digit's first key of this block, minus `start`
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, rank = (int)blockIdx.x;
+    const int per = ((n + kClWarps * 32 - 1) / (kClWarps * 32)) * 32;  // keys per warp, at most 32 ITEMS
+    const int b0 = min(n, rank * kW * per), bn = min(n - b0, kW * per);  // this block's keys
+    const int wn = max(0, min(bn - w * per, per));                       // this warp's
+    uint64_t *ks = keys, *kd = tk;
+    for (int shift = bit_lo; shift < 64; shift += 8) {
+        for (int d = threadIdx.x; d < kW * 256; d += kClThreads) wh[d] = 0;
+        uint64_t key[ITEMS];
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j)
+            key[j] = 32 * j + lane < wn ? __ldcg(ks + b0 + w * per + 32 * j + lane) : 0;
+        __syncthreads();
+        uint32_t rank2[(ITEMS + 1) / 2];
+        warp_ranks<ITEMS>(key, per, wn, shift, wh + w * 256, rank2);
+        __syncthreads();
+        if (threadIdx.x < 256) {
+            const int d = threadIdx.x;
+            int32_t run = 0;
+#pragma unroll
+            for (int q = 0; q < kW; ++q) {
+                const int32_t t = wh[q * 256 + d];
+                wh[q * 256 + d] = run;
+                run += t;
+            }
+            tot[d] = run;
+        }
+        cluster_barrier();
+        int32_t before = 0, all = 0, own = 0;
+        if (threadIdx.x < 256) {
+            own = tot[threadIdx.x];
+#pragma unroll
+            for (int r = 0; r < kClBlocks; ++r) {
+                const int32_t t = cluster_load(&tot[threadIdx.x], r);
+                all += t;
+                before += r < rank ? t : 0;
+            }
+        }
+        const int32_t base = block_excl_scan(all, nullptr), first = block_excl_scan(own, nullptr);
+        if (threadIdx.x < 256) {
+            start[threadIdx.x] = first;
+            out[threadIdx.x] = base + before - first;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j) {
+            const int d = (int)((key[j] >> shift) & 255);
+            if (32 * j + lane < wn)
+                tile[start[d] + wh[w * 256 + d] + (int)((rank2[j / 2] >> (16 * (j % 2))) & 0xffffu)] = key[j];
+        }
+        __syncthreads();
+        const bool last = shift + 8 >= 64;
+        for (int i = threadIdx.x; i < bn; i += kClThreads) {
+            const uint64_t k = tile[i];
+            const int pos = out[(int)((k >> shift) & 255)] + i;
+            kd[pos] = k;
+            if (last) perm[pos] = (int32_t)(uint32_t)k;
+        }
+        cluster_barrier();  // this pass's output is complete, and every block has read the others' totals
+        uint64_t* const kt = ks;
+        ks = kd;
+        kd = kt;
+    }
+    if (ks != keys)  // an odd number of passes
+        for (int i = rank * kClThreads + threadIdx.x; i < n; i += kClBlocks * kClThreads) keys[i] = __ldcg(ks + i);
+}
+
+// One scatter pass over packed keys, many blocks: a tile of kSortTile keys per block, `offsets` (digit-major, scanned)
+// its digits' global positions.  perm, if not null (the last pass), receives the indices.
+__global__ void __launch_bounds__(kSortThreads) packed_scatter_kernel(const uint64_t* __restrict__ kin,
+                                                                      uint64_t* __restrict__ kout,
+                                                                      int32_t* __restrict__ perm, int64_t n, int shift,
+                                                                      const int32_t* __restrict__ offsets,
+                                                                      int nblocks) {
+    constexpr int kW = kSortThreads / 32, kPer = kSortTile / kW, kI = kSortItems;
+    static_assert(kPer == 32 * kI && kSortThreads == 256, "a warp's segment is kSortItems keys per lane");
+    __shared__ uint64_t tile[kSortTile];
+    __shared__ int32_t wh[kW][256], start[256], out[256];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int d = threadIdx.x; d < kW * 256; d += kSortThreads) (&wh[0][0])[d] = 0;
+    const int64_t b0 = (int64_t)blockIdx.x * kSortTile;
+    const int bn = (int)min((int64_t)kSortTile, n - b0), wn = max(0, min(bn - w * kPer, kPer));
+    uint64_t key[kI];
+#pragma unroll
+    for (int j = 0; j < kI; ++j) key[j] = 32 * j + lane < wn ? kin[b0 + w * kPer + 32 * j + lane] : 0;
+    __syncthreads();
+    uint32_t rank2[(kI + 1) / 2];
+    warp_ranks<kI>(key, kPer, wn, shift, wh[w], rank2);
+    __syncthreads();
+    int32_t run = 0;
+    {
+        const int d = threadIdx.x;
+#pragma unroll
+        for (int q = 0; q < kW; ++q) {
+            const int32_t t = wh[q][d];
+            wh[q][d] = run;
+            run += t;
+        }
+    }
+    const int32_t first = block_excl_scan(run, nullptr);
+    start[threadIdx.x] = first;
+    out[threadIdx.x] = offsets[(int64_t)threadIdx.x * nblocks + blockIdx.x] - first;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kI; ++j) {
+        const int d = (int)((key[j] >> shift) & 255);
+        if (32 * j + lane < wn) tile[start[d] + wh[w][d] + (int)((rank2[j / 2] >> (16 * (j % 2))) & 0xffffu)] = key[j];
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < bn; i += kSortThreads) {
+        const uint64_t k = tile[i];
+        const int pos = out[(int)((k >> shift) & 255)] + i;
+        kout[pos] = k;
+        if (perm) perm[pos] = (int32_t)(uint32_t)k;
+    }
+}
+
+// Digit counts of every tile to global offsets; a single block suffices for small arrays, the three-pass scan takes
+// the large ones (1.3M keys: 256 x 320 counts).
+int digit_offsets(lpm_ctx* ctx, int32_t* counts, int64_t m, int sums_slot) {
+    if (m > 16 * 1024) return scan_exclusive_i32(ctx, counts, counts, m, nullptr, sums_slot);
+    LPM_LAUNCH(ctx, "scan_single_block_kernel", scan_single_block_kernel, 1, 1024, 0, counts, m, (int32_t*)nullptr);
+    return LPM_OK;
+}
+
+template <int ITEMS>
+int cluster_sort(lpm_ctx* ctx, uint64_t* keys, uint64_t* tk, int32_t* perm, int64_t n, int bit_lo) {
+    constexpr size_t smem = ClusterSortShape<ITEMS>::kSmem;
+    LPM_CUDA_TRY(cudaFuncSetAttribute(cluster_sort_kernel<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)smem));
+    LPM_LAUNCH(ctx, "cluster_sort_kernel", cluster_sort_kernel<ITEMS>, kClBlocks, kClThreads, smem, keys, tk, perm,
+               (int)n, bit_lo);
+    return LPM_OK;
+}
+
+constexpr int64_t kClusterSortMax = 16 * kClBlocks * kClThreads;
+
 template <typename K>
 int radix_sort_impl(lpm_ctx* ctx, K* keys, int32_t* vals, K* tk, int32_t* tv, int64_t n, int bit_lo, int bit_hi,
                     int counts_slot, int sums_slot) {
@@ -191,15 +417,8 @@ int radix_sort_impl(lpm_ctx* ctx, K* keys, int32_t* vals, K* tk, int32_t* tv, in
     for (int shift = bit_lo; shift < bit_hi; shift += 8) {
         LPM_LAUNCH(ctx, "radix_hist_kernel", radix_hist_kernel<K>, nblocks, kSortThreads, 0, src_k, n, shift, counts,
                    nblocks);
-        // digit-major counts -> global offsets; a single block suffices for small arrays, the three-pass
-        // scan takes the large ones (1.3M keys: 256 x 1280 counts)
-        if ((int64_t)256 * nblocks <= 16 * 1024) {
-            LPM_LAUNCH(ctx, "scan_single_block_kernel", scan_single_block_kernel, 1, 1024, 0, counts,
-                       (int64_t)256 * nblocks, (int32_t*)nullptr);
-        } else {
-            const int rc = scan_exclusive_i32(ctx, counts, counts, (int64_t)256 * nblocks, nullptr, sums_slot);
-            if (rc) return rc;
-        }
+        const int rc = digit_offsets(ctx, counts, (int64_t)256 * nblocks, sums_slot);
+        if (rc) return rc;
         LPM_LAUNCH(ctx, "radix_scatter_kernel", radix_scatter_kernel<K>, nblocks, kSortThreads, 0, src_k, src_v, dst_k,
                    dst_v, n, shift, counts, nblocks);
         std::swap(src_k, dst_k);
@@ -215,7 +434,7 @@ int radix_sort_impl(lpm_ctx* ctx, K* keys, int32_t* vals, K* tk, int32_t* tv, in
 // ---------------------------------------------------------------------------------- keys
 __global__ void morton_keys_kernel(const double4* __restrict__ pts, int64_t n, RootBox root,
                                    uint64_t* __restrict__ keys, int32_t* __restrict__ vals,
-                                   int32_t* __restrict__ counters, int bits, int max_depth) {
+                                   int32_t* __restrict__ counters, int bits, int max_depth, bool packed) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     root = resolve_root(root);
     bool in = false;
@@ -258,8 +477,12 @@ __global__ void morton_keys_kernel(const double4* __restrict__ pts, int64_t n, R
                 key |= digit << (3 * (kKeyLevels - l));
             }
         }
-        keys[i] = key;
-        vals[i] = (int32_t)i;
+        if (packed) {
+            keys[i] = (key & ~0xffffffffull) | (uint64_t)i;
+        } else {
+            keys[i] = key;
+            vals[i] = (int32_t)i;
+        }
     }
     const unsigned b = __ballot_sync(0xffffffffu, in);
     if ((threadIdx.x & 31) == 0 && b) atomicAdd(&counters[0], __popc(b));
@@ -320,168 +543,244 @@ __device__ bool box_meets_sphere(const double* b, double r) {
     return mag3(c[0], c[1], c[2]) <= r && far >= r;
 }
 
-__global__ void tree_init_kernel(Octree t) {
-    t.node_start[0] = 0;
-    t.node_end[0] = t.counters[0];
-    t.node_parent[0] = -1;
-    t.node_first_child[0] = -1;
-    t.node_nchild[0] = 0;
-    t.node_level[0] = 0;
-    const RootBox root = resolve_root(t.root);
-    for (int a = 0; a < 3; ++a) {
-        t.node_box[2 * a] = root.lo[a];
-        t.node_box[2 * a + 1] = root.hi[a];
+// The first position in [s, e) of the sorted keys whose level-l digit is >= d (e if there is none).
+__device__ __forceinline__ int digit_bound(const uint64_t* __restrict__ keys, int s, int e, int l, int d, int bits) {
+    while (s < e) {
+        const int mid = (s + e) >> 1;
+        if (level_digit(keys[mid], l, bits) < d) s = mid + 1;
+        else e = mid;
     }
-    t.level_range[0] = 0;
-    t.level_range[1] = 1;
-    for (int l = 1; l < kMaxLevels + 2; ++l) {
-        t.level_range[2 * l] = 1;
-        t.level_range[2 * l + 1] = 1;
-    }
-    t.counters[1] = 1;
-    t.counters[2] = 0;
-    t.counters[4] = 0;
+    return s;
 }
-
-// For each node of level l holding more than max_per_leaf points: the 9 boundaries of its
-// level-(l+1) digit ranges, and the number of non-empty children.
-__global__ void __launch_bounds__(256) split_level_kernel(Octree t, int l) {
-    // One block per node (grid-stride over the level): warp d (1..7) finds the first position of the node's
-    // sorted key range whose level-(l+1) digit is >= d by a 32-ary search (32 probes per round, ~4 rounds
-    // for a million keys instead of ~20 dependent probes of a binary search).
-    __shared__ int cs_sh[9];
-    const int lb = t.level_range[2 * l], le = t.level_range[2 * l + 1];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+// The same found by a whole warp: a 32-ary search (32 probes per round, ~4 rounds for a million keys instead of ~20
+// dependent probes of a binary search).
+__device__ __forceinline__ int digit_bound_warp(const uint64_t* __restrict__ keys, int s, int e, int l, int d,
+                                                int bits) {
+    const int lane = threadIdx.x & 31;
     const unsigned full = 0xffffffffu;
+    int lo = s, hi = e;  // the boundary b satisfies lo <= b <= hi; positions lo..hi-1 are keys
+    while (hi - lo > 32) {
+        const int64_t L = hi - lo;
+        const int p = lo + (int)(((int64_t)lane * L) >> 5);
+        const unsigned below = __ballot_sync(full, level_digit(keys[p], l, bits) < d);
+        const int c = __popc(below);  // probes 0..c-1 lie below the boundary (digits are sorted)
+        const int nlo = c == 0 ? lo : lo + (int)(((int64_t)(c - 1) * L) >> 5) + 1;
+        const int nhi = c == 32 ? hi : lo + (int)(((int64_t)c * L) >> 5);
+        lo = nlo;
+        hi = nhi;
+    }
+    const bool less = lane < hi - lo && level_digit(keys[lo + lane], l, bits) < d;
+    return lo + __popc(__ballot_sync(full, less));
+}
+
+// The nodes of the sorted keys, level by level, and the leaf numbering, by one cluster.  A level takes two steps: the
+// boundaries of every split node's child digits (one warp per boundary while the level has few nodes, one thread
+// per boundary after), then the child counts' prefix sum (block totals through distributed shared memory) and the
+// children.  Levels stop at the first that splits no node.  Then, level by level again, the leaves below every node
+// are counted upwards and numbered downwards: leaves in depth-first order are numbered by their nodes' order, no
+// pass over the points.  `pending`, if not null, receives every node's number of internal children.
+__global__ void __cluster_dims__(kClBlocks, 1, 1) __launch_bounds__(kClThreads)
+    tree_nodes_kernel(Octree t, int32_t* __restrict__ pending) {
+    __shared__ int32_t slot[2];
+    __shared__ int32_t level_begin[kMaxLevels + 3];
+    const int rank = (int)blockIdx.x, tid = rank * kClThreads + (int)threadIdx.x, lane = threadIdx.x & 31;
+    constexpr int kAll = kClBlocks * kClThreads;
     const int nd = 1 << t.bits;  // digits per level
-    for (int i = lb + blockIdx.x; i < le; i += gridDim.x) {
-        const int s = t.node_start[i], e = t.node_end[i];
-        const bool split = e - s > t.max_per_leaf;  // uniform per block
-        if (split) {
-            if (w >= 1 && w < nd) {
-                const int d = w;
-                int lo = s, hi = e;  // the boundary b satisfies lo <= b <= hi; positions lo..hi-1 are keys
-                while (hi - lo > 32) {
-                    const int64_t L = hi - lo;
-                    const int p = lo + (int)(((int64_t)lane * L) >> 5);
-                    const unsigned below = __ballot_sync(full, level_digit(t.keys[p], l + 1, t.bits) < d);
-                    const int c = __popc(below);  // probes 0..c-1 lie below the boundary (digits are sorted)
-                    const int nlo = c == 0 ? lo : lo + (int)(((int64_t)(c - 1) * L) >> 5) + 1;
-                    const int nhi = c == 32 ? hi : lo + (int)(((int64_t)c * L) >> 5);
-                    lo = nlo;
-                    hi = nhi;
-                }
-                const bool lt = lane < hi - lo && level_digit(t.keys[lo + lane], l + 1, t.bits) < d;
-                const int c = __popc(__ballot_sync(full, lt));
-                if (lane == 0) cs_sh[d] = lo + c;
-            } else if (w == 0 && lane == 0) {
-                cs_sh[0] = s;
-                cs_sh[nd] = e;
-            }
+    const int n_valid = t.counters[0];
+    if (tid == 0) {
+        t.node_start[0] = 0;
+        t.node_end[0] = n_valid;
+        t.node_parent[0] = -1;
+        t.node_first_child[0] = -1;
+        t.node_nchild[0] = 0;
+        t.node_level[0] = 0;
+        const RootBox root = resolve_root(t.root);
+        for (int a = 0; a < 3; ++a) {
+            t.node_box[2 * a] = root.lo[a];
+            t.node_box[2 * a + 1] = root.hi[a];
         }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int nchild = 0;
-            if (split) {
-                int32_t* cs = t.child_start + (int64_t)(i - lb) * 9;
-                for (int d = 0; d <= nd; ++d) cs[d] = cs_sh[d];
-                for (int d = 0; d < nd; ++d) {
-                    bool keep = cs_sh[d + 1] > cs_sh[d];
-                    if (keep && t.sphere_r > 0.0) {
-                        double cb[6];
-                        child_box(t.node_box + 6 * (int64_t)i, l, d, t.bits, cb);
-                        keep = box_meets_sphere(cb, t.sphere_r);
-                    }
-                    nchild += keep;
-                }
-            }
-            t.node_split[i - lb] = nchild;
-        }
-        __syncthreads();  // cs_sh is reused by the next node
     }
-}
-
-// One block: scan the level's child counts and append the children as level l+1.
-__global__ void emit_level_kernel(Octree t, int l) {
-    __shared__ int32_t s_total;
-    const int lb = t.level_range[2 * l], le = t.level_range[2 * l + 1];
-    const int m = le - lb;
-    const int per = (m + blockDim.x - 1) / blockDim.x;
-    const int b = threadIdx.x * per, e = min(b + per, m);
-    int32_t s = 0;
-    for (int i = b; i < e; ++i) s += t.node_split[i];
-    int32_t tot;
-    int32_t run = block_excl_scan(s, &tot) + le;
-    if (threadIdx.x == 0) s_total = tot;
-    for (int i = b; i < e; ++i) {
-        const int node = lb + i;
-        const int nc = t.node_split[i];
-        if (nc == 0 || run + nc > t.node_cap) {
-            if (nc > 0) atomicOr(&t.counters[2], 2);  // node capacity exhausted
-            t.node_first_child[node] = -1;
-            t.node_nchild[node] = 0;
-            continue;
-        }
-        t.node_first_child[node] = run;
-        t.node_nchild[node] = (int8_t)nc;
-        const int32_t* cs = t.child_start + (int64_t)i * 9;
-        const double* pb = t.node_box + 6 * (int64_t)node;
-        int k = run;
-        for (int d = 0; d < (1 << t.bits); ++d) {
-            if (cs[d + 1] <= cs[d]) continue;
-            double cb[6];
-            child_box(pb, l, d, t.bits, cb);
-            if (t.sphere_r > 0.0 && !box_meets_sphere(cb, t.sphere_r)) continue;  // as counted by split_level
-            t.node_start[k] = cs[d];
-            t.node_end[k] = cs[d + 1];
-            t.node_parent[k] = node;
-            t.node_first_child[k] = -1;
-            t.node_nchild[k] = 0;
-            t.node_level[k] = (int8_t)(l + 1);
-            for (int a = 0; a < 6; ++a) t.node_box[6 * (int64_t)k + a] = cb[a];
-            ++k;
-        }
-        run += nc;
-    }
-    __syncthreads();
     if (threadIdx.x == 0) {
-        const int tot2 = (int)min((int64_t)s_total, t.node_cap - (int64_t)le);
-        t.level_range[2 * (l + 1)] = le;
-        t.level_range[2 * (l + 1) + 1] = le + max(tot2, 0);
-        t.counters[1] = le + max(tot2, 0);
-        if (tot2 > 0) t.counters[4] = l + 1;
+        level_begin[0] = 0;
+        level_begin[1] = 1;
     }
-}
-
-__global__ void leaf_flags_kernel(Octree t, int64_t n) {
-    const int nn = t.counters[1];
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += gridDim.x * blockDim.x) {
-        if (t.node_nchild[i] == 0) {
-            t.leaf_flag[t.node_start[i]] = 1;
-            if (t.max_per_leaf > 0 && t.node_end[i] - t.node_start[i] > t.max_per_leaf)
-                atomicOr(&t.counters[2], 1);  // depth limit
-        }
-    }
-    (void)n;
-}
-
-__global__ void leaf_ids_kernel(Octree t, int64_t n) {
-    const int nn = t.counters[1];
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += gridDim.x * blockDim.x) {
-        if (t.node_nchild[i] == 0) {
-            const int leaf = t.leaf_flag[t.node_start[i]];
-            t.node_leaf[i] = leaf;
-            t.leaf_node[leaf] = i;
+    int lb = 0, le = 1, depth = 0;
+    int32_t flags = 0;
+    cluster_barrier();
+    for (int l = 0; l < t.max_depth; ++l) {
+        const int m = le - lb;
+        // boundaries 1 .. nd - 1 of every node that splits
+        if (m * (nd - 1) <= 2 * kClWarps) {
+            for (int q = tid >> 5; q < m * (nd - 1); q += kClWarps) {
+                const int i = q / (nd - 1), d = q - i * (nd - 1) + 1;
+                const int s = __ldcg(t.node_start + lb + i), e = __ldcg(t.node_end + lb + i);
+                if (e - s > t.max_per_leaf) {  // warp-uniform
+                    const int at = digit_bound_warp(t.keys, s, e, l + 1, d, t.bits);
+                    if (lane == 0) t.child_start[(int64_t)i * 9 + d] = at;
+                }
+            }
         } else {
-            t.node_leaf[i] = -1;
+            for (int64_t q = tid; q < (int64_t)m * (nd - 1); q += kAll) {
+                const int i = (int)(q / (nd - 1)), d = (int)(q - (int64_t)i * (nd - 1)) + 1;
+                const int s = __ldcg(t.node_start + lb + i), e = __ldcg(t.node_end + lb + i);
+                if (e - s > t.max_per_leaf)
+                    t.child_start[(int64_t)i * 9 + d] = digit_bound(t.keys, s, e, l + 1, d, t.bits);
+            }
+        }
+        cluster_barrier();
+        // child counts of this block's nodes, block by block in node order, and their prefix sum
+        const int chunk = (m + kClBlocks - 1) / kClBlocks, cb = min(m, rank * chunk), ce = min(m, cb + chunk);
+        const int per = (ce - cb + kClThreads - 1) / kClThreads;
+        const int b = min(ce, cb + (int)threadIdx.x * per), e = min(ce, b + per);
+        // the boundaries of node lb + i in cs[0 .. nd]; the kept children, as bits
+        auto children = [&](int i, int* cs) -> unsigned {
+            const int s = __ldcg(t.node_start + lb + i), en = __ldcg(t.node_end + lb + i);
+            if (en - s <= t.max_per_leaf) return 0u;
+            cs[0] = s;
+            cs[nd] = en;
+            for (int d = 1; d < nd; ++d) cs[d] = __ldcg(t.child_start + (int64_t)i * 9 + d);
+            unsigned keep = 0;
+            for (int d = 0; d < nd; ++d) {
+                if (cs[d + 1] <= cs[d]) continue;
+                if (t.sphere_r > 0.0) {
+                    double pb[6], cbox[6];
+                    for (int a = 0; a < 6; ++a) pb[a] = __ldcg(t.node_box + 6 * (int64_t)(lb + i) + a);
+                    child_box(pb, l, d, t.bits, cbox);
+                    if (!box_meets_sphere(cbox, t.sphere_r)) continue;
+                }
+                keep |= 1u << d;
+            }
+            return keep;
+        };
+        int cs[9];
+        int32_t mine = 0;
+        for (int i = b; i < e; ++i) mine += __popc(children(i, cs));
+        int32_t block_total = 0, total = 0;
+        int32_t run = block_excl_scan(mine, &block_total);
+        run += le + cluster_excl(block_total, &slot[l & 1], rank, &total);
+        const bool fits = (int64_t)le + total <= t.node_cap;
+        if (!fits) flags |= 2;  // node capacity exhausted: the level's nodes stay leaves
+        for (int i = b; i < e && fits; ++i) {
+            const int node = lb + i;
+            const unsigned keep = children(i, cs);
+            const int nc = __popc(keep);
+            if (nc == 0) continue;
+            t.node_first_child[node] = run;
+            t.node_nchild[node] = (int8_t)nc;
+            double pb[6], cbox[6];
+            for (int a = 0; a < 6; ++a) pb[a] = __ldcg(t.node_box + 6 * (int64_t)node + a);
+            int k = run;
+            for (int d = 0; d < nd; ++d) {
+                if (!((keep >> d) & 1u)) continue;
+                child_box(pb, l, d, t.bits, cbox);
+                t.node_start[k] = cs[d];
+                t.node_end[k] = cs[d + 1];
+                t.node_parent[k] = node;
+                t.node_first_child[k] = -1;
+                t.node_nchild[k] = 0;
+                t.node_level[k] = (int8_t)(l + 1);
+                for (int a = 0; a < 6; ++a) t.node_box[6 * (int64_t)k + a] = cbox[a];
+                ++k;
+            }
+            run += nc;
+        }
+        const int next = fits ? total : 0;
+        if (threadIdx.x == 0) level_begin[l + 2] = le + next;
+        lb = le;
+        le += next;
+        cluster_barrier();  // the children are visible to every block
+        if (next == 0) break;  // uniform over the cluster
+        depth = l + 1;
+    }
+    // leaves below every node, upwards
+    for (int l = depth; l >= 0; --l) {
+        for (int node = level_begin[l] + tid; node < level_begin[l + 1]; node += kAll) {
+            const int nc = __ldcg(t.node_nchild + node), fc = __ldcg(t.node_first_child + node);
+            int leaves = nc == 0, internal = 0;
+            for (int k = 0; k < nc; ++k) {
+                leaves += __ldcg(t.node_leaves + fc + k);
+                internal += __ldcg(t.node_nchild + fc + k) > 0;
+            }
+            t.node_leaves[node] = leaves;
+            if (pending) pending[node] = internal;
+        }
+        cluster_barrier();
+    }
+    // leaf numbers, downwards
+    if (tid == 0) t.node_leaf0[0] = 0;
+    for (int l = 0; l <= depth; ++l) {
+        if (l > 0) cluster_barrier();
+        for (int node = level_begin[l] + tid; node < level_begin[l + 1]; node += kAll) {
+            const int nc = __ldcg(t.node_nchild + node);
+            int leaf = l == 0 ? 0 : __ldcg(t.node_leaf0 + node);
+            if (nc == 0) {
+                t.leaf_node[leaf] = node;
+                if (t.max_per_leaf > 0 && __ldcg(t.node_end + node) - __ldcg(t.node_start + node) > t.max_per_leaf)
+                    flags |= 1;  // depth limit
+            }
+            const int fc = __ldcg(t.node_first_child + node);
+            for (int k = 0; k < nc; ++k) {
+                t.node_leaf0[fc + k] = leaf;
+                leaf += __ldcg(t.node_leaves + fc + k);
+            }
         }
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) t.counters[3] = t.leaf_flag[n];
+    if (flags) atomicOr(&t.counters[2], flags);
+    if (tid == 0) {
+        t.counters[1] = le;
+        t.counters[3] = t.n_points > 0 ? __ldcg(t.node_leaves) : 0;
+        t.counters[4] = depth;
+    }
+    cluster_barrier();  // no block leaves while another reads its shared memory
 }
 
-__global__ void fill_i32_kernel(int32_t* p, int64_t n, int32_t v) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = v;
+// Batch starts of n <= kClusterSortMax sorted keys by one cluster (the rule of batch_flags_kernel and
+// batch_first_kernel, treecode.cu): batches start every `batch` positions from the first key of each cell
+// (keys >> shift).  Every thread walks a run of consecutive positions, the first one's cell start found by binary search.
+__global__ void __cluster_dims__(kClBlocks, 1, 1) __launch_bounds__(kClThreads)
+    batch_cut_kernel(const uint64_t* __restrict__ keys, int n, int shift, int batch, int32_t* __restrict__ batch_first,
+                     int32_t* __restrict__ nbat, int64_t cap) {
+    __shared__ int32_t slot;
+    const int rank = (int)blockIdx.x, tid = rank * kClThreads + (int)threadIdx.x;
+    constexpr int kAll = kClBlocks * kClThreads;
+    const int per = (n + kAll - 1) / kAll, b = (int)min((int64_t)n, (int64_t)tid * per), e = min(n, b + per);
+    int pos0 = 0;
+    if (b < e) {
+        const uint64_t cell = keys[b] >> shift;
+        int lo = 0, hi = b;  // smallest j <= b in the same cell
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if ((keys[mid] >> shift) < cell) lo = mid + 1;
+            else hi = mid;
+        }
+        pos0 = (b - lo) % batch;
+    }
+    auto walk = [&](auto start) {  // start(q) at every batch start of the thread's run
+        int pos = pos0;
+        uint64_t cell = b < e ? keys[b] >> shift : 0;
+        for (int q = b; q < e; ++q) {
+            const uint64_t c = keys[q] >> shift;
+            if (c != cell) {
+                cell = c;
+                pos = 0;
+            }
+            if (pos == 0) start(q);
+            if (++pos == batch) pos = 0;
+        }
+    };
+    int32_t count = 0, block_total = 0, total = 0;
+    walk([&](int) { ++count; });
+    int32_t at = block_excl_scan(count, &block_total);
+    at += cluster_excl(block_total, &slot, rank, &total);
+    walk([&](int q) {
+        if (at <= cap) batch_first[at] = q;
+        ++at;
+    });
+    if (tid == 0) {
+        if (total <= cap) batch_first[total] = n;
+        *nbat = total;
+    }
+    cluster_barrier();  // no block leaves while another reads its total
 }
 
 }  // namespace
@@ -498,25 +797,52 @@ int scan_exclusive_i32(lpm_ctx* ctx, const int32_t* in, int32_t* out, int64_t n,
     return LPM_OK;
 }
 
-int morton_keys(lpm_ctx* ctx, const double4* pts, int64_t n, const RootBox& root, uint64_t* keys, int32_t* vals,
-                int32_t* counter) {
+int sort_points(lpm_ctx* ctx, const double4* pts, int64_t n, const RootBox& root, int bits, int max_depth, int bit_lo,
+                uint64_t* keys, int32_t* perm, uint64_t* tk, int32_t* tv, int32_t* counter, int counts_slot,
+                int sums_slot) {
     if (n <= 0) return LPM_OK;
-    LPM_LAUNCH(ctx, "morton_keys_kernel", morton_keys_kernel, grid_for(n, 256), 256, 0, pts, n, root, keys, vals,
-               counter, 3, kKeyLevels);
+    const bool packed = bit_lo >= 32;
+    LPM_LAUNCH(ctx, "morton_keys_kernel", morton_keys_kernel, grid_for(n, 256), 256, 0, pts, n, root, keys, perm, counter,
+               bits, max_depth, packed);
+    if (!packed) return radix_sort_impl<uint64_t>(ctx, keys, perm, tk, tv, n, bit_lo, 64, counts_slot, sums_slot);
+    if (n <= 4 * kClBlocks * kClThreads) return cluster_sort<4>(ctx, keys, tk, perm, n, bit_lo);
+    if (n <= 8 * kClBlocks * kClThreads) return cluster_sort<8>(ctx, keys, tk, perm, n, bit_lo);
+    if (n <= kClusterSortMax) return cluster_sort<16>(ctx, keys, tk, perm, n, bit_lo);
+    const int nblocks = (int)((n + kSortTile - 1) / kSortTile);
+    int32_t* counts = (int32_t*)scratch(ctx, counts_slot, sizeof(int32_t) * 256 * (size_t)nblocks);
+    if (!counts) return LPM_ERR_OOM;
+    uint64_t *ks = keys, *kd = tk;
+    for (int shift = bit_lo; shift < 64; shift += 8) {
+        LPM_LAUNCH(ctx, "radix_hist_kernel", radix_hist_kernel<uint64_t>, nblocks, kSortThreads, 0, ks, n, shift, counts,
+                   nblocks);
+        const int rc = digit_offsets(ctx, counts, (int64_t)256 * nblocks, sums_slot);
+        if (rc) return rc;
+        LPM_LAUNCH(ctx, "packed_scatter_kernel", packed_scatter_kernel, nblocks, kSortThreads, 0, ks, kd,
+                   shift + 8 >= 64 ? perm : nullptr, n, shift, counts, nblocks);
+        std::swap(ks, kd);
+    }
+    if (ks != keys)
+        LPM_CUDA_TRY(cudaMemcpyAsync(keys, ks, sizeof(uint64_t) * (size_t)n, cudaMemcpyDeviceToDevice, ctx->stream));
     return LPM_OK;
 }
 
+bool batch_cut(lpm_ctx* ctx, const uint64_t* keys, int64_t n, int shift, int batch, int32_t* batch_first, int32_t* nbat,
+               int64_t cap, int* rc) {
+    if (n > kClusterSortMax) return false;
+    auto launch = [&]() -> int {
+        LPM_LAUNCH(ctx, "batch_cut_kernel", batch_cut_kernel, kClBlocks, kClThreads, 0, keys, (int)n, shift, batch,
+                   batch_first, nbat, cap);
+        return LPM_OK;
+    };
+    *rc = launch();
+    return true;
+}
+
 int root_extent(lpm_ctx* ctx, const double4* pts, int64_t first, int64_t n, int mode, unsigned long long* r_dev) {
-    LPM_CUDA_TRY(cudaMemsetAsync(r_dev, 0, sizeof(unsigned long long), ctx->stream));
     if (n <= first) return LPM_OK;
     const unsigned g = (unsigned)std::max<int64_t>(1, std::min<int64_t>(grid_for(n - first, 256), 2 * ctx->num_sms));
     LPM_LAUNCH(ctx, "root_extent_kernel", root_extent_kernel, g, 256, 0, pts, first, n, mode, r_dev);
     return LPM_OK;
-}
-
-int radix_sort_u64(lpm_ctx* ctx, uint64_t* keys, int32_t* vals, uint64_t* tk, int32_t* tv, int64_t n, int bit_lo,
-                   int counts_slot, int sums_slot) {
-    return radix_sort_impl<uint64_t>(ctx, keys, vals, tk, tv, n, bit_lo, 64, counts_slot, sums_slot);
 }
 
 int radix_sort_u32(lpm_ctx* ctx, uint32_t* keys, int32_t* vals, uint32_t* tk, int32_t* tv, int64_t n, int bits) {
@@ -551,7 +877,6 @@ int octree_alloc(Octree& t, int64_t n, int max_per_leaf, int max_depth, int bits
     A((void**)&t.perm, nn * 4);
     A((void**)&t.tmp_keys, nn * 8);
     A((void**)&t.tmp_vals, nn * 4);
-    A((void**)&t.leaf_flag, (nn + 1) * 4);
     A((void**)&t.node_start, nc * 4);
     A((void**)&t.node_end, nc * 4);
     A((void**)&t.node_parent, nc * 4);
@@ -559,12 +884,11 @@ int octree_alloc(Octree& t, int64_t n, int max_per_leaf, int max_depth, int bits
     A((void**)&t.node_nchild, nc);
     A((void**)&t.node_level, nc);
     A((void**)&t.node_box, nc * 6 * 8);
-    A((void**)&t.node_split, nc * 4);
     A((void**)&t.child_start, nc * 9 * 4);
-    A((void**)&t.level_range, 2 * (kMaxLevels + 2) * 4);
     A((void**)&t.counters, 16 * 4);
     A((void**)&t.leaf_node, nc * 4);
-    A((void**)&t.node_leaf, nc * 4);
+    A((void**)&t.node_leaf0, nc * 4);
+    A((void**)&t.node_leaves, nc * 4);
     if (e != cudaSuccess) {
         octree_free(t);
         return cuda_status(e, "cudaMalloc (octree)");
@@ -573,9 +897,9 @@ int octree_alloc(Octree& t, int64_t n, int max_per_leaf, int max_depth, int bits
 }
 
 void octree_free(Octree& t) {
-    void* ps[] = {t.keys, t.perm, t.tmp_keys, t.tmp_vals, t.leaf_flag, t.node_start, t.node_end, t.node_parent,
-                  t.node_first_child, t.node_nchild, t.node_level, t.node_box, t.node_split, t.child_start,
-                  t.level_range, t.counters, t.leaf_node, t.node_leaf};
+    void* ps[] = {t.keys, t.perm, t.tmp_keys, t.tmp_vals, t.node_start, t.node_end, t.node_parent,
+                  t.node_first_child, t.node_nchild, t.node_level, t.node_box, t.child_start, t.counters, t.leaf_node,
+                  t.node_leaf0, t.node_leaves};
     for (void* p : ps)
         if (p) cudaFree(p);
     const Octree keep = t;
@@ -588,33 +912,20 @@ void octree_free(Octree& t) {
     t.sphere_r = keep.sphere_r;
 }
 
-int octree_build(lpm_ctx* ctx, Octree& t, const double4* pts, int64_t n, const RootBox& root) {
+int octree_build(lpm_ctx* ctx, Octree& t, const double4* pts, int64_t n, const RootBox& root, int32_t* pending) {
     if (n > t.n || n >= INT32_MAX) {
         set_error("octree_build: %lld points exceed the tree's capacity", (long long)n);
         return LPM_ERR_CAPACITY;
     }
     t.root = root;
+    t.n_points = n;
     LPM_CUDA_TRY(cudaMemsetAsync(t.counters, 0, 16 * 4, ctx->stream));
-    if (n > 0)
-        LPM_LAUNCH(ctx, "morton_keys_kernel", morton_keys_kernel, grid_for(n, 256), 256, 0, pts, n, root, t.keys,
-                   t.perm, t.counters, t.bits, t.max_depth);
     // the key bits that decide levels 1..max_depth (and the outside flag in bit 63)
     const int bit_lo = std::max(0, t.bits * (t.levels - t.max_depth)) & ~7;
-    int rc = radix_sort_u64(ctx, t.keys, t.perm, t.tmp_keys, t.tmp_vals, n, bit_lo);
+    int rc = sort_points(ctx, pts, n, root, t.bits, t.max_depth, bit_lo, t.keys, t.perm, t.tmp_keys, t.tmp_vals,
+                         t.counters);
     if (rc) return rc;
-    LPM_LAUNCH(ctx, "tree_init_kernel", tree_init_kernel, 1, 1, 0, t);
-    const unsigned sgrid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(grid_for(t.node_cap, 256),
-                                                                             4 * ctx->num_sms));
-    const unsigned split_grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(t.node_cap, 8 * ctx->num_sms));
-    for (int l = 0; l < t.max_depth; ++l) {
-        LPM_LAUNCH(ctx, "split_level_kernel", split_level_kernel, split_grid, 256, 0, t, l);
-        LPM_LAUNCH(ctx, "emit_level_kernel", emit_level_kernel, 1, 1024, 0, t, l);
-    }
-    LPM_LAUNCH(ctx, "fill_i32_kernel", fill_i32_kernel, grid_for(n + 1, 256), 256, 0, t.leaf_flag, n + 1, 0);
-    LPM_LAUNCH(ctx, "leaf_flags_kernel", leaf_flags_kernel, sgrid, 256, 0, t, n);
-    rc = scan_exclusive_i32(ctx, t.leaf_flag, t.leaf_flag, n + 1, nullptr);
-    if (rc) return rc;
-    LPM_LAUNCH(ctx, "leaf_ids_kernel", leaf_ids_kernel, sgrid, 256, 0, t, n);
+    LPM_LAUNCH(ctx, "tree_nodes_kernel", tree_nodes_kernel, kClBlocks, kClThreads, 0, t, pending);
     return LPM_OK;
 }
 

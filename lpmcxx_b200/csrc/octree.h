@@ -14,11 +14,12 @@ constexpr uint64_t kKeyOutside = ~0ull;
 int scan_exclusive_i32(lpm_ctx* ctx, const int32_t* in, int32_t* out, int64_t n, int32_t* total_dev,
                        int sums_slot = kSlotMisc2);
 
-// Stable LSD radix sort of (key, value) pairs over key bits [bit_lo, 64), 8 bits per pass.
-// keys/vals are sorted in place (ping-pong through tmp_keys/tmp_vals, which must hold n items).  Digit counts
-// go to ctx scratch slot `counts_slot`, scan sums to `sums_slot` (sorts on concurrent streams use distinct slots).
-int radix_sort_u64(lpm_ctx* ctx, uint64_t* keys, int32_t* vals, uint64_t* tmp_keys, int32_t* tmp_vals, int64_t n,
-                   int bit_lo, int counts_slot = kSlotMisc1, int sums_slot = kSlotMisc2);
+// Cuts n sorted keys into batches of at most `batch` keys of one cell (keys >> shift): batch_first[0 .. *nbat - 1] their
+// starts, batch_first[*nbat] = n (entries up to index cap), by one launch; false (nothing done) for large n.
+bool batch_cut(lpm_ctx* ctx, const uint64_t* keys, int64_t n, int shift, int batch, int32_t* batch_first, int32_t* nbat,
+               int64_t cap, int* rc);
+// Stable LSD radix sort of (key, value) pairs over key bits [0, bits), 8 bits per pass, in place (ping-pong through
+// tmp_keys / tmp_vals, which must hold n items).
 int radix_sort_u32(lpm_ctx* ctx, uint32_t* keys, int32_t* vals, uint32_t* tmp_keys, int32_t* tmp_vals, int64_t n,
                    int bits);
 
@@ -60,7 +61,8 @@ int root_extent(lpm_ctx* ctx, const double4* pts, int64_t first, int64_t n, int 
 // (max_per_leaf = 0), and with sphere_r > 0 a child is kept only if its box meets the sphere of that radius
 // about the origin (Box3d::intersectsSphere, src/LpmBox3d.cpp:125-129).
 struct Octree {
-    int64_t n = 0;          // points given
+    int64_t n = 0;          // points the arrays hold
+    int64_t n_points = 0;   // points of the last build
     int max_per_leaf = 0;
     int max_depth = 0;      // levels the keys are split to (<= levels)
     int bits = 3;           // key bits per level: 3 (octree) or 1 (binary, axis-cycling)
@@ -81,23 +83,27 @@ struct Octree {
     int8_t* node_nchild = nullptr;
     int8_t* node_level = nullptr;
     double* node_box = nullptr;           // 6 per node: xlo, xhi, ylo, yhi, zlo, zhi
-    int32_t* node_split = nullptr;        // scratch: child counts of a level
     int32_t* child_start = nullptr;       // scratch: 9 boundaries per node of a level
-    int32_t* level_range = nullptr;       // [2 * (kKeyLevels + 2)]: begin/end of each level's nodes
     int32_t* counters = nullptr;          // [0] n_valid, [1] n_nodes, [2] overflow flag, [3] n_leaves, [4] depth
     // leaves in depth-first order
     int32_t* leaf_node = nullptr;         // leaf index -> node id
-    int32_t* node_leaf = nullptr;         // node id -> leaf index (or -1)
-    int32_t* leaf_flag = nullptr;         // scratch over points
+    int32_t* node_leaf0 = nullptr;        // node id -> index of the first leaf at or below it ...
+    int32_t* node_leaves = nullptr;       // ... and their number
 };
 
-// keys[i], vals[i] = i for pts[0:n]; counter[0] += number of points inside the root box.
-int morton_keys(lpm_ctx* ctx, const double4* pts, int64_t n, const RootBox& root, uint64_t* keys, int32_t* vals,
-                int32_t* counter);
+// The Morton keys (replayed bisections of the root box) of pts[0:n], sorted stably over their bits [bit_lo, 64): keys
+// in order, perm[q] the index of the q-th; counter[0] += number of points inside the root box.  With bit_lo >= 32 the
+// keys' lower 32 bits hold the index instead.  tk / tv: n items of scratch; digit counts go to ctx scratch slot
+// `counts_slot`, scan sums to `sums_slot` (sorts on concurrent streams use distinct slots).
+int sort_points(lpm_ctx* ctx, const double4* pts, int64_t n, const RootBox& root, int bits, int max_depth, int bit_lo,
+                uint64_t* keys, int32_t* perm, uint64_t* tk, int32_t* tv, int32_t* counter,
+                int counts_slot = kSlotMisc1, int sums_slot = kSlotMisc2);
 
 int octree_alloc(Octree& t, int64_t n, int max_per_leaf, int max_depth, int bits = 3, double sphere_r = 0.0);
 void octree_free(Octree& t);
-// Build over pts[0:n] with the given root box.  Fully asynchronous (capturable): no host reads.
-int octree_build(lpm_ctx* ctx, Octree& t, const double4* pts, int64_t n, const RootBox& root);
+// Build over pts[0:n] with the given root box.  Fully asynchronous (capturable): no host reads.  `pending` (node_cap
+// ints, may be null) receives every node's number of internal children.
+int octree_build(lpm_ctx* ctx, Octree& t, const double4* pts, int64_t n, const RootBox& root,
+                 int32_t* pending = nullptr);
 
 }  // namespace lpm

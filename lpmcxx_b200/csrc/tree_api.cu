@@ -21,14 +21,21 @@ struct lpm_tree {
 namespace lpm {
 namespace {
 
-__global__ void leaf_of_point_kernel(const int32_t* __restrict__ perm, const int32_t* __restrict__ leaf_scan,
-                                     int64_t n, int64_t n_valid, uint32_t* __restrict__ leaf_key,
-                                     int32_t* __restrict__ idx) {
+// The leaf of every point: the last one (in depth-first order) that starts at or before its sorted position.
+__global__ void leaf_of_point_kernel(const int32_t* __restrict__ perm, const int32_t* __restrict__ leaf_node,
+                                     const int32_t* __restrict__ node_start, int n_leaves, int64_t n, int64_t n_valid,
+                                     uint32_t* __restrict__ leaf_key, int32_t* __restrict__ idx) {
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
     idx[p] = (int32_t)p;  // original indices in increasing order (the values of the stable sort)
     const int32_t orig = perm[p];
-    leaf_key[orig] = p < n_valid ? (uint32_t)(leaf_scan[p + 1] - 1) : 0xffffffffu;
+    int lo = 0, hi = n_leaves;  // leaves before lo start at or before p, leaves from hi on after it
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (node_start[leaf_node[mid]] <= p) lo = mid + 1;
+        else hi = mid;
+    }
+    leaf_key[orig] = p < n_valid ? (uint32_t)(lo - 1) : 0xffffffffu;
 }
 
 }  // namespace
@@ -183,7 +190,7 @@ extern "C" int lpm_tree_leaf_membership(lpm_tree* tr, int64_t* members, int64_t*
     int32_t* tv = (int32_t*)scratch(ctx, kSlotTree3, sizeof(int32_t) * (size_t)n);
     if (!key || !idx || !tk || !tv) return LPM_ERR_OOM;
     LPM_LAUNCH(ctx, "leaf_of_point_kernel", leaf_of_point_kernel, grid_for(n, 256), 256, 0, tr->t.perm,
-               tr->t.leaf_flag, n, tr->n_valid, key, idx);
+               tr->t.leaf_node, tr->t.node_start, (int)tr->n_leaves, n, tr->n_valid, key, idx);
     int rc = radix_sort_u32(ctx, key, idx, tk, tv, n, 32);
     if (rc) return rc;
     std::vector<int32_t> h(n), starts(tr->n_leaves + 1), lnode(tr->n_leaves), nstart(tr->n_nodes);

@@ -247,16 +247,6 @@ __device__ __forceinline__ double4 ldcg4(const double4* p) {
     return make_double4(a.x, a.y, b.x, b.y);
 }
 
-__global__ void m2m_pending_kernel(Octree t, int32_t* __restrict__ pending) {
-    const int nn = t.counters[1];
-    for (int node = blockIdx.x * blockDim.x + threadIdx.x; node < nn; node += gridDim.x * blockDim.x) {
-        const int nc = t.node_nchild[node];
-        int p = 0;
-        for (int k = 0; k < nc; ++k) p += t.node_nchild[t.node_first_child[node] + k] > 0;
-        pending[node] = p;
-    }
-}
-
 constexpr int kM2mThreads = 256;
 __global__ void __launch_bounds__(kM2mThreads) m2m_upward_kernel(Octree t, int pm, const int4* __restrict__ mono,
                                                          int n_mono, double4* __restrict__ node_ctr,
@@ -690,8 +680,8 @@ __global__ void __launch_bounds__(128, LPM_TRAVERSE_MIN_BLOCKS) traverse_kernel(
                 kind = 1;
             } else if (far_ok || nc == 0) {
                 kind = 2;
-                lo = t.leaf_flag[s];
-                hi = t.leaf_flag[e] - 1;
+                lo = t.node_leaf0[node];
+                hi = lo + t.node_leaves[node] - 1;
                 cnt = e - s;
             } else {
                 kind = 3;
@@ -763,41 +753,158 @@ __global__ void __launch_bounds__(128, LPM_TRAVERSE_MIN_BLOCKS) traverse_kernel(
 // that takes batches in this order from an atomic ticket ends on its smallest batches, so few SMs idle at
 // its tail.  Each batch is still computed by one block, so the results do not depend on the order.
 constexpr int kSchedBuckets = 64;
-// the solver's schedule scratch (int32): near buckets and cursors, far buckets and cursors, then one ticket
-// for the near launch and one per far order
-constexpr int kAuxNearHist = 0, kAuxNearCur = 64, kAuxFarHist = 128, kAuxFarCur = 192, kAuxNearTicket = 256,
-              kAuxFarTicket = 257, kAuxInts = 257 + 16;
+// the solver's zero block (int32, cleared by one memset at the start of an evaluation): flags, target counts, pair
+// counters (8-byte), root radius (8-byte), then one ticket for the near launch and one per far order
+constexpr int kZeroFlags = 0, kZeroTcount = 8, kZeroPairs = 12, kZeroRoot = 18, kZeroNearTicket = 20,
+              kZeroFarTicket = 21, kZeroInts = 21 + 16;
 
 __device__ __forceinline__ int sched_bucket(uint32_t work) {
     const int l2 = (int)(2.0f * __log2f((float)work + 1.0f));
     return kSchedBuckets - 1 - min(max(l2, 0), kSchedBuckets - 1);
 }
 
-// hist[0:64] and cursor[0:64] zeroed by the caller.
-__global__ void sched_hist_kernel(const uint32_t* __restrict__ work, const int32_t* __restrict__ nbat,
-                                  int32_t* __restrict__ hist) {
-    const int n = *nbat;
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < n; b += gridDim.x * blockDim.x)
-        atomicAdd(&hist[sched_bucket(work[b])], 1);
-}
+struct ListsArgs {
+    const int32_t* nbat;
+    int64_t nb1;  // row stride of far_cnt / far_off
+    int p_lo, p_hi;  // the far orders present
+    const int32_t* far_cnt;
+    const int32_t* near_cnt;
+    int32_t* far_off;
+    int32_t* near_off;
+    int32_t* totals;  // [0] far entries, [1] near entries
+    int sched;        // also order the batches by decreasing work
+    const uint32_t* far_work;
+    const uint32_t* near_work;
+    int32_t* far_order;
+    int32_t* near_order;
+};
 
-__global__ void sched_scatter_kernel(const uint32_t* __restrict__ work, const int32_t* __restrict__ nbat,
-                                     const int32_t* __restrict__ hist, int32_t* __restrict__ cursor,
-                                     int32_t* __restrict__ order) {
-    __shared__ int base[kSchedBuckets];
-    if (threadIdx.x == 0) {
-        int acc = 0;
-        for (int k = 0; k < kSchedBuckets; ++k) {
-            base[k] = acc;
-            acc += hist[k];
+// After the traversal's count pass, by one thread-block cluster (8 blocks meeting at the hardware barrier): the offsets
+// of every batch's far entries (exclusive prefix sums over the order rows present, row by row) and near entries, and
+// the batches bucketed by decreasing far and near work.  As eleven launches (two three-pass scans over every row and
+// batch slot, two histograms and two scatters) these cost about 45 us of a small evaluation.
+constexpr int kListsBlocks = 8, kListsThreads = 1024;
+__device__ __forceinline__ void lists_barrier() {
+    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;\n" ::: "memory");
+}
+__device__ __forceinline__ int32_t lists_load(const int32_t* p, int rank) {  // the int at p in block `rank`
+    const unsigned s = (unsigned)__cvta_generic_to_shared(p);
+    int32_t v;
+    asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %1, %2;\n\tld.shared::cluster.s32 %0, [ra];\n\t}"
+                 : "=r"(v)
+                 : "r"(s), "r"(rank)
+                 : "memory");
+    return v;
+}
+__global__ void __cluster_dims__(kListsBlocks, 1, 1) __launch_bounds__(kListsThreads) lists_kernel(ListsArgs A) {
+    __shared__ int32_t warp_sums[2][32], block_sum[2];
+    __shared__ int32_t hist[2][kSchedBuckets], bucket[2][kSchedBuckets], cursor[2][kSchedBuckets];
+    const int rank = (int)blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int nbat = *A.nbat;
+    if (threadIdx.x < 2 * kSchedBuckets) (&hist[0][0])[threadIdx.x] = 0;
+    __syncthreads();
+    // this thread's run of consecutive (row, batch) entries of the far counts, and of batches of the near counts
+    const int64_t n_far = (int64_t)(A.p_hi - A.p_lo + 1) * nbat;
+    constexpr int kAll = kListsBlocks * kListsThreads;
+    const int64_t tid = (int64_t)rank * kListsThreads + threadIdx.x;
+    const int64_t fper = (n_far + kAll - 1) / kAll, fb = min(n_far, tid * fper), fe = min(n_far, fb + fper);
+    const int nper = (nbat + kAll - 1) / kAll, nb = (int)min((int64_t)nbat, tid * nper), ne = min(nbat, nb + nper);
+    auto far_run = [&](auto entry) {  // entry(index into far_cnt / far_off) for each of the run
+        if (fb >= fe) return;
+        int row = A.p_lo + (int)(fb / nbat), b = (int)(fb % nbat);
+        for (int64_t k = fb; k < fe; ++k) {
+            entry((int64_t)row * A.nb1 + b);
+            if (++b == nbat) {
+                b = 0;
+                ++row;
+            }
+        }
+    };
+    int32_t far = 0, near = 0;
+    far_run([&](int64_t at) { far += A.far_cnt[at]; });
+    for (int b = nb; b < ne; ++b) near += A.near_cnt[b];
+    if (A.sched)
+        for (int b = (int)tid; b < nbat; b += kAll) {
+            atomicAdd(&hist[0][sched_bucket(A.far_work[b])], 1);
+            atomicAdd(&hist[1][sched_bucket(A.near_work[b])], 1);
+        }
+    // exclusive prefix over the block's threads, then over the blocks
+    int32_t fi = far, ni = near;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int32_t f = __shfl_up_sync(0xffffffffu, fi, o), n = __shfl_up_sync(0xffffffffu, ni, o);
+        if (lane >= o) {
+            fi += f;
+            ni += n;
         }
     }
-    __syncthreads();
-    const int n = *nbat;
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < n; b += gridDim.x * blockDim.x) {
-        const int k = sched_bucket(work[b]);
-        order[base[k] + atomicAdd(&cursor[k], 1)] = b;
+    if (lane == 31) {
+        warp_sums[0][w] = fi;
+        warp_sums[1][w] = ni;
     }
+    __syncthreads();
+    if (w < 2) {
+        int32_t v = warp_sums[w][lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int32_t t = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += t;
+        }
+        warp_sums[w][lane] = v;
+        if (lane == 31) block_sum[w] = v;
+    }
+    __syncthreads();
+    int32_t far_at = fi - far + (w ? warp_sums[0][w - 1] : 0), near_at = ni - near + (w ? warp_sums[1][w - 1] : 0);
+    lists_barrier();
+    int32_t far_all = 0, near_all = 0;
+#pragma unroll
+    for (int r = 0; r < kListsBlocks; ++r) {
+        const int32_t f = lists_load(&block_sum[0], r), n = lists_load(&block_sum[1], r);
+        far_all += f;
+        near_all += n;
+        if (r < rank) {
+            far_at += f;
+            near_at += n;
+        }
+    }
+    if (tid == 0) {
+        A.totals[0] = far_all;
+        A.totals[1] = near_all;
+    }
+    if (A.sched && threadIdx.x < 2 * kSchedBuckets) {  // this block's first slot of each bucket
+        const int q = threadIdx.x / kSchedBuckets, k = threadIdx.x % kSchedBuckets;
+        int32_t all = 0, before = 0;
+#pragma unroll
+        for (int r = 0; r < kListsBlocks; ++r) {
+            const int32_t h = lists_load(&hist[q][k], r);
+            all += h;
+            before += r < rank ? h : 0;
+        }
+        bucket[q][k] = all;
+        cursor[q][k] = before;
+    }
+    __syncthreads();
+    if (A.sched && threadIdx.x < 2 * kSchedBuckets) {
+        const int q = threadIdx.x / kSchedBuckets, k = threadIdx.x % kSchedBuckets;
+        int32_t at = 0;
+        for (int j = 0; j < k; ++j) at += bucket[q][j];
+        cursor[q][k] += at;
+    }
+    __syncthreads();
+    far_run([&](int64_t at) {
+        A.far_off[at] = far_at;
+        far_at += A.far_cnt[at];
+    });
+    for (int b = nb; b < ne; ++b) {
+        A.near_off[b] = near_at;
+        near_at += A.near_cnt[b];
+    }
+    if (A.sched)
+        for (int b = (int)tid; b < nbat; b += kAll) {
+            A.far_order[atomicAdd(&cursor[0][sched_bucket(A.far_work[b])], 1)] = b;
+            A.near_order[atomicAdd(&cursor[1][sched_bucket(A.near_work[b])], 1)] = b;
+        }
+    lists_barrier();  // no block leaves while another reads its sums
 }
 
 // The next batch of a persistent kernel's block: order[ticket++] while tickets last, else -1.  ticket is
@@ -2240,6 +2347,7 @@ struct TreeSolver {
     double root_maxr = 0.0;
     int64_t root_first = 0;
     unsigned long long* root_r = nullptr;
+    int32_t* zero = nullptr;  // kZero* layout: flags, tcount, pair_counts, root_r and the tickets lie in it
     Octree st;
     // target ordering
     uint64_t* tkeys = nullptr;
@@ -2292,7 +2400,6 @@ struct TreeSolver {
     uint32_t* far_work = nullptr;     // per batch: far coefficient evaluations (count pass)
     int32_t* sched_order = nullptr;   // batches by decreasing near work
     int32_t* far_order = nullptr;     // batches by decreasing far work
-    int32_t* sched_aux = nullptr;     // kAux* layout below
     int near_blocks = 1;              // persistent grids: resident blocks on the whole device
     int near_targets = kNearTargets;  // near kernel tile shape (run-time "near_targets", "near_tile")
     int near_tile = kNearStreamTile;
@@ -2528,7 +2635,6 @@ int tree_solver_create(lpm_ctx* ctx, const lpm_kernel_desc& kernel, const lpm_so
     A(talloc(t, &t->tperm, ntg));
     A(talloc(t, &t->ttmpk, ntg));
     A(talloc(t, &t->ttmpv, ntg));
-    A(talloc(t, &t->tcount, 4));
     A(talloc(t, &t->tgt_sorted, ntg));
     A(talloc(t, &t->batch_ctr, (size_t)t->n_batches));
     A(talloc(t, &t->bflag, ntg + 1));
@@ -2562,14 +2668,11 @@ int tree_solver_create(lpm_ctx* ctx, const lpm_kernel_desc& kernel, const lpm_so
     A(talloc(t, &t->near_cnt, (size_t)t->n_batches + 1));
     A(talloc(t, &t->far_off, far_rows));
     A(talloc(t, &t->near_off, (size_t)t->n_batches + 1));
-    A(talloc(t, &t->flags, 8));
-    A(talloc(t, &t->root_r, 1));
+    A(talloc(t, &t->zero, kZeroInts));
     A(talloc(t, &t->near_work, (size_t)t->n_batches + 1));
     A(talloc(t, &t->far_work, (size_t)t->n_batches + 1));
     A(talloc(t, &t->sched_order, (size_t)t->n_batches + 1));
     A(talloc(t, &t->far_order, (size_t)t->n_batches + 1));
-    A(talloc(t, &t->sched_aux, kAuxInts));
-    A(talloc(t, &t->pair_counts, 3));
     A(talloc(t, &t->V, 3 * ntg));
     A(talloc(t, &t->W, scalar ? ntg : 1));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&t->side, cudaStreamNonBlocking);
@@ -2599,6 +2702,10 @@ int tree_solver_create(lpm_ctx* ctx, const lpm_kernel_desc& kernel, const lpm_so
         tree_solver_destroy(t);
         return cuda_status(e, "tree solver allocation");
     }
+    t->flags = t->zero + kZeroFlags;
+    t->tcount = t->zero + kZeroTcount;
+    t->pair_counts = (unsigned long long*)(t->zero + kZeroPairs);
+    t->root_r = (unsigned long long*)(t->zero + kZeroRoot);
     {
         cudaError_t ea = far_smem_attributes();
         // M2M stages two 8-child copies of the moments: opt in for the largest order any solver may use
@@ -2674,7 +2781,14 @@ void tree_solver_destroy(TreeSolver* t) {
     delete t;
 }
 
-static int build_lists(TreeSolver* t, bool can_sync) {
+// The far-field orders of an evaluation: the fixed order, or the selector's orders 1..11.
+static void far_order_range(const TreeSolver* t, int* p_lo, int* p_hi) {
+    const bool sel = t->learned && t->mlp_loaded;
+    *p_lo = sel ? 1 : t->order;
+    *p_hi = sel ? std::min(t->pm, kMlpDirectClass) : t->order;
+}
+
+static int build_lists(TreeSolver* t, bool can_sync, bool sched) {
     lpm_ctx* ctx = t->ctx;
     TraverseArgs A{};
     A.t = t->st;
@@ -2707,13 +2821,24 @@ static int build_lists(TreeSolver* t, bool can_sync) {
     A.heavy_cap = t->heavy_cap;
     A.near_work = t->near_work;
     A.far_work = t->far_work;
-    LPM_CUDA_TRY(cudaMemsetAsync(t->pair_counts, 0, 3 * sizeof(unsigned long long), ctx->stream));
     const unsigned g = grid_for(t->n_batches, 4);
     LPM_LAUNCH(ctx, "traverse_kernel", traverse_kernel, g, 128, 0, A);
-    int rc = scan_exclusive_i32(ctx, t->far_cnt, t->far_off, (int64_t)(kPMax + 1) * (t->n_batches + 1), t->flags + 2);
-    if (rc) return rc;
-    rc = scan_exclusive_i32(ctx, t->near_cnt, t->near_off, t->n_batches + 1, t->flags + 3);
-    if (rc) return rc;
+    ListsArgs L{};
+    L.nbat = t->tcount + 1;
+    L.nb1 = t->n_batches + 1;
+    far_order_range(t, &L.p_lo, &L.p_hi);
+    L.far_cnt = t->far_cnt;
+    L.near_cnt = t->near_cnt;
+    L.far_off = t->far_off;
+    L.near_off = t->near_off;
+    L.totals = t->flags + 2;
+    L.sched = sched ? 1 : 0;
+    L.far_work = t->far_work;
+    L.near_work = t->near_work;
+    L.far_order = t->far_order;
+    L.near_order = t->sched_order;
+    LPM_LAUNCH(ctx, "lists_kernel", lists_kernel, kListsBlocks, kListsThreads, 0, L);
+    int rc = LPM_OK;
     if (can_sync) {
         int32_t tot[2];
         LPM_CUDA_TRY(cudaMemcpyAsync(tot, t->flags + 2, sizeof(tot), cudaMemcpyDeviceToHost, ctx->stream));
@@ -2731,13 +2856,6 @@ static int build_lists(TreeSolver* t, bool can_sync) {
     A.near_cap = t->near_cap;
     LPM_LAUNCH(ctx, "traverse_kernel", traverse_kernel, g, 128, 0, A);
     return LPM_OK;
-}
-
-// The far-field orders of an evaluation: the fixed order, or the selector's orders 1..11.
-static void far_order_range(const TreeSolver* t, int* p_lo, int* p_hi) {
-    const bool sel = t->learned && t->mlp_loaded;
-    *p_lo = sel ? 1 : t->order;
-    *p_hi = sel ? std::min(t->pm, kMlpDirectClass) : t->order;
 }
 
 // Everything of an evaluation before its far and near fields: root box, target batches, source octree, moments,
@@ -2760,7 +2878,7 @@ static int tree_prepare(TreeSolver* t, const double4* src, int64_t n_src, const 
         LPM_CUDA_TRY(cudaMemsetAsync(U, 0, (t->scalar ? 1 : 3) * (size_t)n_tgt * sizeof(double), ctx->stream));
         return LPM_OK;
     }
-    LPM_CUDA_TRY(cudaMemsetAsync(t->flags, 0, 8 * sizeof(int32_t), ctx->stream));
+    LPM_CUDA_TRY(cudaMemsetAsync(t->zero, 0, kZeroInts * sizeof(int32_t), ctx->stream));
     RootBox rb;
     int rc = LPM_OK;
     if (!t->scalar && t->root_maxr > 0.0) {
@@ -2783,20 +2901,23 @@ static int tree_prepare(TreeSolver* t, const double4* src, int64_t n_src, const 
     // scan use their own scratch slots.
     const unsigned gt = (unsigned)std::max<int64_t>(1, std::min<int64_t>(grid_for(n_tgt + 1, 256), 8 * ctx->num_sms));
     auto target_batches = [&]() -> int {
-        LPM_CUDA_TRY(cudaMemsetAsync(t->tcount, 0, 4 * sizeof(int32_t), ctx->stream));
-        int r = morton_keys(ctx, X, n_tgt, rb, t->tkeys, t->tperm, t->tcount);
+        int r = sort_points(ctx, X, n_tgt, rb, 3, kKeyLevels, 32, t->tkeys, t->tperm, t->ttmpk, t->ttmpv, t->tcount,
+                            kSlotSideCounts, kSlotSideSums);
         if (r) return r;
-        r = radix_sort_u64(ctx, t->tkeys, t->tperm, t->ttmpk, t->ttmpv, n_tgt, 32, kSlotSideCounts, kSlotSideSums);
+        const int shift = 3 * (kKeyLevels - t->batch_level);
+        if (!batch_cut(ctx, t->tkeys, n_tgt, shift, kBatch, t->batch_first, t->tcount + 1, t->n_batches, &r)) {
+            LPM_CUDA_TRY(cudaMemsetAsync(t->bflag + n_tgt, 0, sizeof(int32_t), ctx->stream));
+            LPM_LAUNCH(ctx, "batch_flags_kernel", batch_flags_kernel, gt, 256, 0, t->tkeys, n_tgt, shift, t->bflag);
+            r = scan_exclusive_i32(ctx, t->bflag, t->bflag, n_tgt + 1, nullptr, kSlotSideSums);
+            if (r) return r;
+            LPM_LAUNCH(ctx, "batch_first_kernel", batch_first_kernel, gt, 256, 0, t->bflag, n_tgt, t->batch_first,
+                       t->tcount + 1, t->n_batches);
+        }
         if (r) return r;
-        LPM_CUDA_TRY(cudaMemsetAsync(t->bflag + n_tgt, 0, sizeof(int32_t), ctx->stream));
-        LPM_LAUNCH(ctx, "batch_flags_kernel", batch_flags_kernel, gt, 256, 0, t->tkeys, n_tgt,
-                   3 * (kKeyLevels - t->batch_level), t->bflag);
-        r = scan_exclusive_i32(ctx, t->bflag, t->bflag, n_tgt + 1, nullptr, kSlotSideSums);
-        if (r) return r;
-        LPM_LAUNCH(ctx, "batch_first_kernel", batch_first_kernel, gt, 256, 0, t->bflag, n_tgt, t->batch_first,
-                   t->tcount + 1, t->n_batches);
         LPM_LAUNCH(ctx, "batch_kernel", batch_kernel, (unsigned)t->n_batches, kBatch, 0, X, t->tperm,
                    t->batch_first, t->tcount + 1, t->tgt_sorted, t->batch_ctr);
+        // the far launches add to V
+        LPM_CUDA_TRY(cudaMemsetAsync(t->V, 0, (t->scalar ? 1 : 3) * (size_t)n_tgt * sizeof(double), ctx->stream));
         return LPM_OK;
     };
     const bool tside = !ctx->profiling;
@@ -2810,7 +2931,7 @@ static int tree_prepare(TreeSolver* t, const double4* src, int64_t n_src, const 
         if (rc) return rc;
         LPM_CUDA_TRY(cudaEventRecord(t->ev_tjoin, t->side));
     }
-    rc = octree_build(ctx, t->st, src, n_src, rb);
+    rc = octree_build(ctx, t->st, src, n_src, rb, t->m2m_pending);
     if (rc) return rc;
     if (can_sync) {  // grow the per-node arrays to this tree (a captured replay can only flag an overflow)
         int32_t nodes = 0;
@@ -2829,7 +2950,6 @@ static int tree_prepare(TreeSolver* t, const double4* src, int64_t n_src, const 
     LPM_LAUNCH(ctx, "leaf_p2m_kernel", leaf_p2m_kernel, gl, kP2mThreads, 0, t->st, t->src_sorted, t->pm, t->p2m_units,
                t->n_units,
                t->node_ctr, t->node_wabs, t->node_mom, t->src32, t->scalar ? 1.0 : 2.0, t->heavy_cap);
-    LPM_LAUNCH(ctx, "m2m_pending_kernel", m2m_pending_kernel, gl, 128, 0, t->st, t->m2m_pending);
     LPM_LAUNCH(ctx, "m2m_upward_kernel", m2m_upward_kernel, gl, kM2mThreads, (size_t)16 * t->n_mono * sizeof(double), t->st,
                t->pm, t->mono, t->n_mono, t->node_ctr, t->node_wabs, t->node_mom, t->heavy_cap, t->m2m_pending);
     // far-field coefficients: needed only by the far kernels, so (profiling off) on the side stream during the
@@ -2865,27 +2985,10 @@ static int tree_prepare(TreeSolver* t, const double4* src, int64_t n_src, const 
         rc = target_batches();
         if (rc) return rc;
     }
-    rc = build_lists(t, can_sync);
+    rc = build_lists(t, can_sync, sched);
     if (rc) return rc;
     if (tside) LPM_CUDA_TRY(cudaStreamWaitEvent(ctx->stream, t->ev_cjoin, 0));  // the coefficients
-    // far field: one launch per order present (only the fixed order, or the selector's orders 1..11),
-    // each adding its bucket's contributions to V
-    LPM_CUDA_TRY(cudaMemsetAsync(t->V, 0, 3 * (size_t)n_tgt * sizeof(double), ctx->stream));
     *pending = true;
-    if (!sched) return LPM_OK;
-    // batch schedules: far and near work of every batch (from the traversal's count pass), bucketed in
-    // decreasing order; zeroed buckets, cursors and tickets first
-    LPM_CUDA_TRY(cudaMemsetAsync(t->sched_aux, 0, kAuxInts * sizeof(int32_t), ctx->stream));
-    const unsigned gsch = (unsigned)std::max<int64_t>(1, std::min<int64_t>(grid_for(t->n_batches, 256),
-                                                                            2 * ctx->num_sms));
-    LPM_LAUNCH(ctx, "sched_hist_kernel", sched_hist_kernel, gsch, 256, 0, t->far_work, t->tcount + 1,
-               t->sched_aux + kAuxFarHist);
-    LPM_LAUNCH(ctx, "sched_scatter_kernel", sched_scatter_kernel, gsch, 256, 0, t->far_work, t->tcount + 1,
-               t->sched_aux + kAuxFarHist, t->sched_aux + kAuxFarCur, t->far_order);
-    LPM_LAUNCH(ctx, "sched_hist_kernel", sched_hist_kernel, gsch, 256, 0, t->near_work, t->tcount + 1,
-               t->sched_aux + kAuxNearHist);
-    LPM_LAUNCH(ctx, "sched_scatter_kernel", sched_scatter_kernel, gsch, 256, 0, t->near_work, t->tcount + 1,
-               t->sched_aux + kAuxNearHist, t->sched_aux + kAuxNearCur, t->sched_order);
     return LPM_OK;
 }
 
@@ -2908,7 +3011,7 @@ static FarArgs far_args(const TreeSolver* t, int P) {
     F.gtab = t->gtab + t->ct.table_off[P];
     F.V = t->V;
     F.order = t->far_order;
-    F.ticket = t->sched_aux + kAuxFarTicket + P;
+    F.ticket = t->zero + kZeroFarTicket + P;
     return F;
 }
 
@@ -2931,7 +3034,7 @@ static NearArgs near_args(const TreeSolver* t, double* U) {
     N.mult = -1.0 / (4.0 * kPi * t->kernel.radius);
     N.U = U;
     N.order = t->sched_order;
-    N.ticket = t->sched_aux + kAuxNearTicket;
+    N.ticket = t->zero + kZeroNearTicket;
     return N;
 }
 
@@ -2953,7 +3056,7 @@ static int tree_far_order(TreeSolver* t, int P) {
             int threads = 0;
             FarKernelFn fn = far_split_select(part, &smem, &threads);
             F.gtab = t->gtab + t->ct.table_off[P] + (part == 2 ? part_entries(P, 1) : 0);
-            F.ticket = t->sched_aux + kAuxFarTicket + (part == 2 ? kPMax + 1 : P);
+            F.ticket = t->zero + kZeroFarTicket + (part == 2 ? kPMax + 1 : P);
             LPM_LAUNCH(ctx, "far_kernel", fn, (unsigned)t->far_split_blocks[part - 1], threads, smem, F);
         }
     } else {
@@ -2995,7 +3098,7 @@ int tree_velocity(TreeSolver* t, const double4* src, int64_t n_src, const double
         FarLowArgs LA{};
         for (int P = p_lo; P <= low_hi; ++P) LA.a[P - 1] = far_args(t, P);
         LPM_LAUNCH(ctx, "far_kernel", far_low2_kernel, (unsigned)t->far_low_blocks, kFar2Threads, far_low_smem(), LA,
-                   t->tcount + 1, t->far_order, t->sched_aux + kAuxFarTicket + p_lo);
+                   t->tcount + 1, t->far_order, t->zero + kZeroFarTicket + p_lo);
         p_lo = low_hi + 1;
     }
     for (int P = p_lo; P <= p_hi; ++P) {
