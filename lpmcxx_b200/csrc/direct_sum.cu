@@ -97,19 +97,6 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-__device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;\n" ::: "memory");
-}
-// The double at `p` of this block's shared memory, read from the block of rank `rank` of the cluster.
-__device__ __forceinline__ double cluster_load(const double* p, int rank) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(p);
-    double v;
-    asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %1, %2;\n\tld.shared::cluster.f64 %0, [ra];\n\t}"
-                 : "=d"(v)
-                 : "r"(s), "r"(rank)
-                 : "memory");
-    return v;
-}
 
 // The threads have left their sums in red[group][target][component][thread of the group]: adds them over the groups
 // and the cluster's blocks and hands each target (in block order u = target * (threads per group) + thread) to
@@ -688,34 +675,6 @@ Split32 split32(int sms, int64_t n_tgt, int64_t n_src, int max_tpt) {
     return best;
 }
 
-// Launch a direct-sum kernel of `blocks` target blocks as clusters of sp.parts blocks.
-template <class... KArgs, class... Args>
-int launch_split(lpm_ctx* ctx, const char* name, void (*kern)(KArgs...), int64_t blocks, int threads, size_t smem, Split sp,
-                 Args... args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)(blocks * sp.parts));
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = ctx->stream;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = (unsigned)sp.parts;
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = sp.parts > 1 ? 1 : 0;
-    LpmProfRecord rec{name, nullptr, nullptr};
-    if (ctx->profiling) prof_begin(ctx, rec);
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
-    if (ctx->profiling) prof_end(ctx, rec);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        return cuda_status(e, name);
-    }
-    ctx->launches += 1;
-    return LPM_OK;
-}
-
 // Whether the vector and 1/r kernels take two targets per thread instead of four: while four leave less than two
 // blocks to an SM even in eight parts (1,280 sources x 1,922 targets: 12.4 against 16.5 us; 5,120 x 7,682: 60.0
 // against 57.5 us).
@@ -729,8 +688,8 @@ int launch64(lpm_ctx* ctx, const char* name, Op op, const double4* src, int64_t 
     const size_t smem = Shape64<Op>::kSmem;
     if (smem > 48 * 1024)
         LPM_CUDA_TRY(cudaFuncSetAttribute(direct64_kernel<Op>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    return launch_split(ctx, name, direct64_kernel<Op>, blocks, kThreads64, smem, sp, src, n_src, tgt, n_tgt, op, mult,
-                        out, stride, coinc_n, coinc_off, sp);
+    return launch_cluster(ctx, name, direct64_kernel<Op>, (unsigned)(blocks * sp.parts), kThreads64, smem, sp.parts, src,
+                          n_src, tgt, n_tgt, op, mult, out, stride, coinc_n, coinc_off, sp);
 }
 
 template <class Op, int TPT>
@@ -739,8 +698,8 @@ int launch32(lpm_ctx* ctx, const char* name, Op op, const float4* src, int64_t n
              int64_t coinc_off, Split sp) {
     const int64_t tb = (kThreads * TPT) >> sp.gshift;
     const size_t smem = std::max(2 * sizeof(float4) * (kTile << sp.gshift), sizeof(double) * kThreads * TPT * Op::NC);
-    return launch_split(ctx, name, direct32_kernel<Op, TPT>, (n_tgt + tb - 1) / tb, kThreads, smem, sp, src, n_src, tgt,
-                        tgt64, n_tgt, op, mult, out, stride, coinc_n, coinc_off, sp);
+    return launch_cluster(ctx, name, direct32_kernel<Op, TPT>, (unsigned)((n_tgt + tb - 1) / tb * sp.parts), kThreads, smem,
+                          sp.parts, src, n_src, tgt, tgt64, n_tgt, op, mult, out, stride, coinc_n, coinc_off, sp);
 }
 }  // namespace
 

@@ -126,6 +126,34 @@ cudaError_t dev_alloc(void** p, size_t bytes);
 void prof_begin(lpm_ctx* ctx, LpmProfRecord& r);
 void prof_end(lpm_ctx* ctx, LpmProfRecord& r);
 
+// LPM_LAUNCH of `blocks` blocks in clusters of `cluster` (a divisor of blocks, at most 8).
+template <class... KArgs, class... Args>
+int launch_cluster(lpm_ctx* ctx, const char* name, void (*kern)(KArgs...), unsigned blocks, int threads, size_t smem,
+                   int cluster, Args... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)cluster;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = cluster > 1 ? 1 : 0;
+    LpmProfRecord rec{name, nullptr, nullptr};
+    if (ctx->profiling) prof_begin(ctx, rec);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+    if (ctx->profiling) prof_end(ctx, rec);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return cuda_status(e, name);
+    }
+    ctx->launches += 1;
+    return LPM_OK;
+}
+
 inline unsigned grid_for(int64_t n, int per_block) { return (unsigned)((n + per_block - 1) / per_block); }
 
 // direct sums (direct_sum.cu)
@@ -141,6 +169,30 @@ int direct_sum_any(lpm_ctx* ctx, const lpm_kernel_desc& k, int precision, const 
 int pack_f32(lpm_ctx* ctx, const double4* in, int64_t n, float4* out, bool scale_w2);
 int check_kernel_desc(const lpm_kernel_desc* k);
 int check_f32_kind(const lpm_kernel_desc& k);  // LPM_ERR_KERNEL unless Biot-Savart or 3D Poisson
+
+// Thread-block clusters: a hardware barrier of all their threads (release / acquire at cluster scope, so it orders global
+// memory too), and the other blocks' shared memory at this block's addresses.
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;\n" ::: "memory");
+}
+__device__ __forceinline__ unsigned cluster_address(const void* p, int rank) {
+    unsigned a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ double cluster_load(const double* p, int rank) {
+    double v;
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(cluster_address(p, rank)) : "memory");
+    return v;
+}
+__device__ __forceinline__ int32_t cluster_load(const int32_t* p, int rank) {
+    int32_t v;
+    asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(cluster_address(p, rank)) : "memory");
+    return v;
+}
+__device__ __forceinline__ void cluster_store(int32_t* p, int rank, int32_t v) {
+    asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(cluster_address(p, rank)), "r"(v) : "memory");
+}
 
 // Packed FP32 (fma.rn.f32x2, sm_100): two FP32 FMAs in one instruction, each lane rounded like fmaf.
 // (d0, d1) = (a0 b + c0, a1 b + c1).

@@ -112,21 +112,6 @@ constexpr int kClBlocks = 8;  // portable cluster size
 constexpr int kClThreads = 1024;
 constexpr int kClWarps = kClBlocks * kClThreads / 32;
 
-// Every thread of the cluster's blocks; orders their memory accesses (release / acquire at cluster scope).
-__device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;\n" ::: "memory");
-}
-// The int at `p` of this block's shared memory, read from the block of rank `rank`.
-__device__ __forceinline__ int32_t cluster_load(const int32_t* p, int rank) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(p);
-    int32_t v;
-    asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %1, %2;\n\tld.shared::cluster.s32 %0, [ra];\n\t}"
-                 : "=r"(v)
-                 : "r"(s), "r"(rank)
-                 : "memory");
-    return v;
-}
-
 // The block's total v over all blocks (*total) and over the blocks of lower rank (returned).  One cluster barrier
 // inside; `slot` (one int of shared memory) may be written again only after the next one.
 __device__ __forceinline__ int32_t cluster_excl(int32_t v, int32_t* slot, int rank, int32_t* total) {

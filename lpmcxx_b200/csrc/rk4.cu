@@ -138,7 +138,10 @@ uint64_t rk4_buffer_generation(const lpm_rk4* rk) {
 }
 lpm_ctx* rk4_context(lpm_rk4* rk) { return rk->ctx; }
 int rk4_tree_check(lpm_rk4* rk) { return rk->tree ? tree_check(rk->tree) : LPM_OK; }
-void rk4_set_owner(lpm_rk4* rk, lpm_ensemble* e) { rk->owner = e; }
+void rk4_set_owner(lpm_rk4* rk, lpm_ensemble* e) {
+    rk->owner = e;
+    if (rk->tree) tree_set_clusters(rk->tree, false);
+}
 int rk4_set_param_internal(lpm_rk4* rk, const char* name, double value) {
     if (!rk->tree) {
         set_error("ensemble: the instances do not use the treecode");

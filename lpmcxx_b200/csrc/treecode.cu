@@ -787,18 +787,6 @@ struct ListsArgs {
 // the batches bucketed by decreasing far and near work.  As eleven launches (two three-pass scans over every row and
 // batch slot, two histograms and two scatters) these cost about 45 us of a small evaluation.
 constexpr int kListsBlocks = 8, kListsThreads = 1024;
-__device__ __forceinline__ void lists_barrier() {
-    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;\n" ::: "memory");
-}
-__device__ __forceinline__ int32_t lists_load(const int32_t* p, int rank) {  // the int at p in block `rank`
-    const unsigned s = (unsigned)__cvta_generic_to_shared(p);
-    int32_t v;
-    asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %1, %2;\n\tld.shared::cluster.s32 %0, [ra];\n\t}"
-                 : "=r"(v)
-                 : "r"(s), "r"(rank)
-                 : "memory");
-    return v;
-}
 __global__ void __cluster_dims__(kListsBlocks, 1, 1) __launch_bounds__(kListsThreads) lists_kernel(ListsArgs A) {
     __shared__ int32_t warp_sums[2][32], block_sum[2];
     __shared__ int32_t hist[2][kSchedBuckets], bucket[2][kSchedBuckets], cursor[2][kSchedBuckets];
@@ -858,11 +846,11 @@ __global__ void __cluster_dims__(kListsBlocks, 1, 1) __launch_bounds__(kListsThr
     }
     __syncthreads();
     int32_t far_at = fi - far + (w ? warp_sums[0][w - 1] : 0), near_at = ni - near + (w ? warp_sums[1][w - 1] : 0);
-    lists_barrier();
+    cluster_barrier();
     int32_t far_all = 0, near_all = 0;
 #pragma unroll
     for (int r = 0; r < kListsBlocks; ++r) {
-        const int32_t f = lists_load(&block_sum[0], r), n = lists_load(&block_sum[1], r);
+        const int32_t f = cluster_load(&block_sum[0], r), n = cluster_load(&block_sum[1], r);
         far_all += f;
         near_all += n;
         if (r < rank) {
@@ -880,7 +868,7 @@ __global__ void __cluster_dims__(kListsBlocks, 1, 1) __launch_bounds__(kListsThr
         int32_t all = 0, before = 0;
 #pragma unroll
         for (int r = 0; r < kListsBlocks; ++r) {
-            const int32_t h = lists_load(&hist[q][k], r);
+            const int32_t h = cluster_load(&hist[q][k], r);
             all += h;
             before += r < rank ? h : 0;
         }
@@ -908,7 +896,7 @@ __global__ void __cluster_dims__(kListsBlocks, 1, 1) __launch_bounds__(kListsThr
             A.far_order[atomicAdd(&cursor[0][sched_bucket(A.far_work[b])], 1)] = b;
             A.near_order[atomicAdd(&cursor[1][sched_bucket(A.near_work[b])], 1)] = b;
         }
-    lists_barrier();  // no block leaves while another reads its sums
+    cluster_barrier();  // no block leaves while another reads its sums
 }
 
 // The next batch of a persistent kernel's block: order[ticket++] while tickets last, else -1.  ticket is
@@ -921,6 +909,27 @@ __device__ __forceinline__ int next_batch(int32_t* ticket, const int32_t* __rest
     }
     __syncthreads();
     return *slot;
+}
+
+// Split launches: a cluster of `parts` blocks takes a batch together, each block every parts-th stage or tile of its
+// list, and block 0 adds their FP64 sums in rank order and writes the result (the FP32 sums of a stage or tile are
+// formed whole in one block, so they are those of the unsplit launch).  For problems of few batches, where one block a
+// batch leaves most of the device idle behind the longest batches.
+struct ClusterPart {
+    int rank, parts;
+};
+// The cluster's next batch, in every block: as next_batch, taken by block 0.  slot[2]: two rounds' worth, so that a
+// block may read the last round's while block 0 stores the next.
+__device__ __forceinline__ int next_batch_split(int32_t* ticket, const int32_t* __restrict__ order, int nbat,
+                                                int32_t* slot, int round, ClusterPart cp) {
+    __syncthreads();
+    if (cp.rank == 0 && threadIdx.x == 0) {
+        const int k = atomicAdd(ticket, 1);
+        const int b = k < nbat ? order[k] : -1;
+        for (int r = 0; r < cp.parts; ++r) cluster_store(slot + (round & 1), r, b);
+    }
+    cluster_barrier();
+    return slot[round & 1];
 }
 
 // ---------------------------------------------------------------------------------- far field
@@ -1338,12 +1347,13 @@ __device__ __forceinline__ void far2_stage_gather(const FarArgs& A, int64_t s0, 
 
 // One batch b of the far2 kernel (the whole block); fbuf: 2 stages of S::kStage units, then 2 x kK centres
 // (FP32 offsets).
-template <int P, int PART = 0>
-__device__ __forceinline__ void far2_batch(const FarArgs& A, int64_t b, float4* fbuf) {
+template <int P, int PART = 0, bool kSplit = false>
+__device__ __forceinline__ void far2_batch(const FarArgs& A, int64_t b, float4* fbuf, ClusterPart cp = {0, 1}) {
     using S = FarShape<P, float4, kFar2StageUnits, PART>;
     float4* ctr = fbuf + 2 * S::kStage;
     const int64_t f0 = A.far_off[b], f1 = min(f0 + (int64_t)A.far_cnt[b], A.far_cap);
-    if (f0 >= f1) return;  // uniform per block
+    if (f0 >= f1) return;  // uniform per block (and cluster)
+    const int64_t step = kSplit ? (int64_t)S::kK * cp.parts : S::kK, first = kSplit ? f0 + (int64_t)S::kK * cp.rank : f0;
     const int64_t q0 = A.batch_first[b], qe = A.batch_first[b + 1];
     // warp w holds targets 64 w .. 64 w + 63 of the batch (lane l: 64 w + l and 64 w + l + 32), so a warp past
     // the batch's last target idles as a whole (batches average ~109 of 128 targets)
@@ -1358,12 +1368,12 @@ __device__ __forceinline__ void far2_batch(const FarArgs& A, int64_t b, float4* 
         xo[t][0] = (float)(p.x - o.x); xo[t][1] = (float)(p.y - o.y); xo[t][2] = (float)(p.z - o.z);
     }
     double acc[2][3] = {{0, 0, 0}, {0, 0, 0}};
-    far2_stage_gather<P, PART>(A, f0, (int)min((int64_t)S::kK, f1 - f0), fbuf, ctr, o);
+    if (!kSplit || first < f1) far2_stage_gather<P, PART>(A, first, (int)min((int64_t)S::kK, f1 - first), fbuf, ctr, o);
     cp_async_commit();
     int s = 0;
-    for (int64_t s0 = f0;; s ^= 1) {
+    for (int64_t s0 = first; !kSplit || s0 < f1; s ^= 1) {
         const int n = (int)min((int64_t)S::kK, f1 - s0);
-        const int64_t s1 = s0 + n;
+        const int64_t s1 = kSplit ? s0 + step : s0 + n;
         if (s1 < f1)
             far2_stage_gather<P, PART>(A, s1, (int)min((int64_t)S::kK, f1 - s1), fbuf + (size_t)(s ^ 1) * S::kStage,
                                  ctr + (s ^ 1) * S::kK, o);
@@ -1384,6 +1394,25 @@ __device__ __forceinline__ void far2_batch(const FarArgs& A, int64_t b, float4* 
         if (s1 >= f1) break;
         __syncthreads();  // stage s consumed before it is refilled
         s0 = s1;
+    }
+    if constexpr (kSplit) {  // block 0 adds the blocks' sums in rank order
+        double* red = reinterpret_cast<double*>(fbuf);
+        __syncthreads();  // the last stage is consumed
+        if (cp.rank > 0)
+#pragma unroll
+            for (int t = 0; t < 2; ++t)
+#pragma unroll
+                for (int c = 0; c < 3; ++c) red[(t * 3 + c) * kFar2Threads + threadIdx.x] = acc[t][c];
+        cluster_barrier();
+        if (cp.rank == 0)
+            for (int r = 1; r < cp.parts; ++r)
+#pragma unroll
+                for (int t = 0; t < 2; ++t)
+#pragma unroll
+                    for (int c = 0; c < 3; ++c)
+                        acc[t][c] += cluster_load(red + (t * 3 + c) * kFar2Threads + threadIdx.x, r);
+        cluster_barrier();  // the sums are read before their space is filled again
+        if (cp.rank > 0) return;
     }
 #pragma unroll
     for (int t = 0; t < 2; ++t) {  // V += 2 x cross (sum of h), x the FP64 target
@@ -1411,6 +1440,20 @@ __global__ void __launch_bounds__(kFar2Threads, kFar2MinBlocks) far_order2_kerne
         far2_batch<P, PART>(A, b, fbuf);
 }
 
+template <int P, int PART = 0>
+__global__ void __launch_bounds__(kFar2Threads, kFar2MinBlocks) far_order2_split_kernel(FarArgs A, int parts) {
+    extern __shared__ float4 fbuf[];
+    __shared__ int32_t slot[2];
+    const ClusterPart cp{(int)(blockIdx.x % (unsigned)parts), parts};
+    const int nbat = *A.nbat;
+    cluster_barrier();  // every block of the cluster runs before another touches its shared memory
+    for (int round = 0;; ++round) {
+        const int64_t b = next_batch_split(A.ticket, A.order, nbat, slot, round, cp);
+        if (b < 0) break;
+        far2_batch<P, PART, true>(A, b, fbuf, cp);
+    }
+}
+
 // The short orders 1..kFarLowMax of the FP32 far field in one persistent launch: a block takes a batch (in
 // decreasing order of its far work) and runs the order-P body for each of these orders in turn, so V receives
 // the orders' sums in the order of separate launches (bitwise the same).  As separate launches these orders
@@ -1436,6 +1479,25 @@ __global__ void __launch_bounds__(kFar2Threads, kFar2MinBlocks) far_low2_kernel(
         if (L.a[2].far_cnt) far2_batch<3>(L.a[2], b, fbuf);
         __syncthreads();
         if (L.a[3].far_cnt) far2_batch<4>(L.a[3], b, fbuf);
+    }
+}
+
+__global__ void __launch_bounds__(kFar2Threads, kFar2MinBlocks) far_low2_split_kernel(FarLowArgs L,
+                                                                                     const int32_t* __restrict__ nbat_p,
+                                                                                     const int32_t* __restrict__ order,
+                                                                                     int32_t* ticket, int parts) {
+    extern __shared__ float4 fbuf[];
+    __shared__ int32_t slot[2];
+    const ClusterPart cp{(int)(blockIdx.x % (unsigned)parts), parts};
+    const int nbat = *nbat_p;
+    cluster_barrier();  // every block of the cluster runs before another touches its shared memory
+    for (int round = 0;; ++round) {  // every far2_batch with work ends in a cluster barrier
+        const int64_t b = next_batch_split(ticket, order, nbat, slot, round, cp);
+        if (b < 0) break;
+        if (L.a[0].far_cnt) far2_batch<1, 0, true>(L.a[0], b, fbuf, cp);
+        if (L.a[1].far_cnt) far2_batch<2, 0, true>(L.a[1], b, fbuf, cp);
+        if (L.a[2].far_cnt) far2_batch<3, 0, true>(L.a[2], b, fbuf, cp);
+        if (L.a[3].far_cnt) far2_batch<4, 0, true>(L.a[3], b, fbuf, cp);
     }
 }
 
@@ -1534,8 +1596,8 @@ constexpr int kFar2ScalarMaxOrder = LPM_FAR2_SCALAR_MAX_ORDER;  // FP32 scalar o
 // T targets per thread (targets i, i + 128/T, ...; T = 2 only in FP32); each entry's contiguous
 // coefficient row (stride entries, 16-byte aligned) is staged with cp.async, kK entries per stage,
 // double-buffered.  Adds sum w/|x - y| to V[q].
-template <int P, typename F, int T>
-__global__ void __launch_bounds__(kBatch / T) far_scalar_kernel(FarArgs A, int stride) {
+template <int P, typename F, int T, bool kSplit>
+__global__ void __launch_bounds__(kBatch / T) far_scalar_kernel(FarArgs A, int stride, int parts) {
     constexpr int kNT = kBatch / T;
     constexpr int kU = T == 2 ? kFar2StageUnits : kFarStageUnits;
     constexpr int kE = entries_for(P);
@@ -1544,11 +1606,17 @@ __global__ void __launch_bounds__(kBatch / T) far_scalar_kernel(FarArgs A, int s
     static_assert(T == 1 || (T == 2 && sizeof(F) == 4), "two targets per thread in FP32 only");
     extern __shared__ float4 fbuf[];  // 2 stages of kK x kUnits units, then 2 x kK centres
     double4* ctr = (double4*)(fbuf + 2 * kK * kUnits);
-    __shared__ int slot;
+    __shared__ int32_t slot[2];
     const int nbat = *A.nbat;
-    for (int64_t b = next_batch(A.ticket, A.order, nbat, &slot); b >= 0; b = next_batch(A.ticket, A.order, nbat, &slot)) {
+    const ClusterPart cp = kSplit ? ClusterPart{(int)(blockIdx.x % (unsigned)parts), parts} : ClusterPart{0, 1};
+    if constexpr (kSplit) cluster_barrier();  // every block of the cluster runs before another touches its shared memory
+    for (int round = 0;; ++round) {
+    const int64_t b = kSplit ? next_batch_split(A.ticket, A.order, nbat, slot, round, cp)
+                             : next_batch(A.ticket, A.order, nbat, slot);
+    if (b < 0) break;
     const int64_t f0 = A.far_off[b], f1 = min(f0 + (int64_t)A.far_cnt[b], A.far_cap);
-    if (f0 >= f1) continue;  // uniform per block
+    if (f0 >= f1) continue;  // uniform per block (and cluster)
+    const int64_t first = f0 + (int64_t)kK * cp.rank, step = (int64_t)kK * cp.parts;
     const int64_t q0 = A.batch_first[b], qe = A.batch_first[b + 1];
     // warp w holds targets 32 T w .. 32 T (w + 1) - 1 of the batch (lane l: 32 T w + l + 32 t), so a warp past
     // the batch's last target idles as a whole
@@ -1586,12 +1654,12 @@ __global__ void __launch_bounds__(kBatch / T) far_scalar_kernel(FarArgs A, int s
     double acc[T];
 #pragma unroll
     for (int t = 0; t < T; ++t) acc[t] = 0.0;
-    gather(f0, (int)min((int64_t)kK, f1 - f0), fbuf, 0);
+    if (!kSplit || first < f1) gather(first, (int)min((int64_t)kK, f1 - first), fbuf, 0);
     cp_async_commit();
     int sb = 0;
-    for (int64_t s0 = f0;; sb ^= 1) {
+    for (int64_t s0 = first; !kSplit || s0 < f1; sb ^= 1) {
         const int n = (int)min((int64_t)kK, f1 - s0);
-        const int64_t s1 = s0 + n;
+        const int64_t s1 = kSplit ? s0 + step : s0 + n;
         if (s1 < f1) gather(s1, (int)min((int64_t)kK, f1 - s1), fbuf + (size_t)(sb ^ 1) * kK * kUnits, sb ^ 1);
         cp_async_commit();
         cp_async_wait_prev();
@@ -1633,16 +1701,30 @@ __global__ void __launch_bounds__(kBatch / T) far_scalar_kernel(FarArgs A, int s
         __syncthreads();  // stage sb consumed before it is refilled
         s0 = s1;
     }
+    if constexpr (kSplit) {  // block 0 adds the blocks' sums in rank order
+        double* red = reinterpret_cast<double*>(fbuf);
+        __syncthreads();  // the last stage is consumed
+        if (cp.rank > 0)
 #pragma unroll
-    for (int t = 0; t < T; ++t)
-        if (q + 32 * t < qe) A.V[q + 32 * t] += acc[t];
+            for (int t = 0; t < T; ++t) red[t * kNT + threadIdx.x] = acc[t];
+        cluster_barrier();
+        if (cp.rank == 0)
+            for (int r = 1; r < cp.parts; ++r)
+#pragma unroll
+                for (int t = 0; t < T; ++t) acc[t] += cluster_load(red + t * kNT + threadIdx.x, r);
+        cluster_barrier();  // the sums are read before their space is filled again
+    }
+    if (cp.rank == 0)
+#pragma unroll
+        for (int t = 0; t < T; ++t)
+            if (q + 32 * t < qe) A.V[q + 32 * t] += acc[t];
     }
 }
 
-typedef void (*FarScalarFn)(FarArgs, int);
+typedef void (*FarScalarFn)(FarArgs, int, int);
 
 template <int P>
-FarScalarFn far_scalar_for(bool f64, size_t* smem, int* threads) {
+FarScalarFn far_scalar_for(bool f64, bool split, size_t* smem, int* threads) {
     constexpr int kE = entries_for(P);
     auto sm = [](int bytes, int U) {
         const int units = (kE * bytes + 15) / 16;
@@ -1652,31 +1734,32 @@ FarScalarFn far_scalar_for(bool f64, size_t* smem, int* threads) {
     *threads = kBatch;
     if (f64) {
         *smem = sm(8, kFarStageUnits);
-        return far_scalar_kernel<P, double, 1>;
+        return split ? nullptr : far_scalar_kernel<P, double, 1, false>;
     }
     if constexpr (P <= kFar2ScalarMaxOrder) {
         *threads = kBatch / 2;
         *smem = sm(4, kFar2StageUnits);
-        return far_scalar_kernel<P, float, 2>;
+        return split ? far_scalar_kernel<P, float, 2, true> : far_scalar_kernel<P, float, 2, false>;
     }
     *smem = sm(4, kFarStageUnits);
-    return far_scalar_kernel<P, float, 1>;
+    return split ? nullptr : far_scalar_kernel<P, float, 1, false>;
 }
 
-FarScalarFn far_scalar_select(int P, bool f64, size_t* smem, int* threads) {
+// The order-P scalar far kernel; split: the cluster launch (FP32 only, else nullptr).
+FarScalarFn far_scalar_select(int P, bool f64, bool split, size_t* smem, int* threads) {
     switch (P) {
-        case 1: return far_scalar_for<1>(f64, smem, threads);
-        case 2: return far_scalar_for<2>(f64, smem, threads);
-        case 3: return far_scalar_for<3>(f64, smem, threads);
-        case 4: return far_scalar_for<4>(f64, smem, threads);
-        case 5: return far_scalar_for<5>(f64, smem, threads);
-        case 6: return far_scalar_for<6>(f64, smem, threads);
-        case 7: return far_scalar_for<7>(f64, smem, threads);
-        case 8: return far_scalar_for<8>(f64, smem, threads);
-        case 9: return far_scalar_for<9>(f64, smem, threads);
-        case 10: return far_scalar_for<10>(f64, smem, threads);
-        case 11: return far_scalar_for<11>(f64, smem, threads);
-        default: return far_scalar_for<12>(f64, smem, threads);
+        case 1: return far_scalar_for<1>(f64, split, smem, threads);
+        case 2: return far_scalar_for<2>(f64, split, smem, threads);
+        case 3: return far_scalar_for<3>(f64, split, smem, threads);
+        case 4: return far_scalar_for<4>(f64, split, smem, threads);
+        case 5: return far_scalar_for<5>(f64, split, smem, threads);
+        case 6: return far_scalar_for<6>(f64, split, smem, threads);
+        case 7: return far_scalar_for<7>(f64, split, smem, threads);
+        case 8: return far_scalar_for<8>(f64, split, smem, threads);
+        case 9: return far_scalar_for<9>(f64, split, smem, threads);
+        case 10: return far_scalar_for<10>(f64, split, smem, threads);
+        case 11: return far_scalar_for<11>(f64, split, smem, threads);
+        default: return far_scalar_for<12>(f64, split, smem, threads);
     }
 }
 
@@ -1696,6 +1779,27 @@ FarKernelFn far_kernel_for(bool f64, size_t* smem, int* threads) {
     }
     *smem = FarShape<P, float4>::kSmem;
     return far_order_kernel<P, float, float4>;
+}
+
+// The cluster launch of the FP32 order-P far kernel (part 1 or 2 at kFarSplitOrder), P <= kFar2MaxOrder; block size and
+// shared memory are far_order2_kernel's.
+typedef void (*FarSplitFn)(FarArgs, int);
+FarSplitFn far_cluster_select(int P, int part) {
+    static_assert(kFar2MaxOrder == 11 && kFarSplitOrder == 11, "cluster far orders 1..11");
+    switch (P) {
+        case 1: return far_order2_split_kernel<1>;
+        case 2: return far_order2_split_kernel<2>;
+        case 3: return far_order2_split_kernel<3>;
+        case 4: return far_order2_split_kernel<4>;
+        case 5: return far_order2_split_kernel<5>;
+        case 6: return far_order2_split_kernel<6>;
+        case 7: return far_order2_split_kernel<7>;
+        case 8: return far_order2_split_kernel<8>;
+        case 9: return far_order2_split_kernel<9>;
+        case 10: return far_order2_split_kernel<10>;
+        case 11: return part == 2 ? far_order2_split_kernel<11, 2> : far_order2_split_kernel<11, 1>;
+        default: return nullptr;
+    }
 }
 
 // The two launches of the FP32 far field at kFarSplitOrder (parts 1 and 2).
@@ -1958,11 +2062,12 @@ struct NearArgs {
 // gives each source read from shared memory to KT targets while keeping two warps on a batch), and the
 // groups' sums are added in shared memory at the end of the batch.  Instances for KT in {2, 4}, KTILE in
 // {256, 512, 1024} and KS in {1, 2} are chosen at run time.
-template <bool kScalar, int KT, int KTILE, int KS>
-__device__ __forceinline__ void near_batch(const NearArgs& A, int64_t b) {
+template <bool kScalar, int KT, int KTILE, int KS, bool kSplit = false>
+__device__ __forceinline__ void near_batch(const NearArgs& A, int64_t b, ClusterPart cp = {0, 1}) {
     constexpr int kT = KT, kTT = kBatch / KT, kThreads = kTT * KS, kNW = kThreads / 32, kRPT = kNearRuns / kThreads;
     static_assert(kT % 2 == 0 && kTT % 32 == 0 && kNearRuns % kThreads == 0, "near kernel shape");
     static_assert((KS - 1) * 3 * kBatch * sizeof(double) <= sizeof(float4) * KTILE, "group sums fit one tile");
+    static_assert(3 * kBatch * sizeof(double) <= sizeof(float4) * KTILE, "block sums fit one tile");
     __shared__ __align__(16) float4 tile[2][KTILE];  // double-buffered: tile p + 1 arrives while p is summed
     __shared__ int r_start[kNearRuns], r_pre[kNearRuns + 1];
     __shared__ int warp_tot[kNW];
@@ -1994,6 +2099,7 @@ __device__ __forceinline__ void near_batch(const NearArgs& A, int64_t b) {
     const int64_t n0 = near_off[b], n1 = min(n0 + (int64_t)near_cnt[b], near_cap);
     const int64_t n_all = n1 - n0;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int turn = cp.rank;  // split: tiles until this block's next one
     for (int64_t c0 = 0; c0 < n_all; c0 += kNearRuns) {
         // resolve up to kNearRuns entries into source ranges and their prefix offsets
         int len[kRPT], st[kRPT];
@@ -2050,11 +2156,12 @@ __device__ __forceinline__ void near_batch(const NearArgs& A, int64_t b) {
             }
         };
         int buf = 0;
-        if (total > 0) stage(0, 0);
+        const int first = kSplit ? turn * KTILE : 0, step = kSplit ? cp.parts * KTILE : KTILE;
+        if (first < total) stage(first, 0);
         cp_async_commit();
-        for (int p0 = 0; p0 < total; p0 += KTILE, buf ^= 1) {
+        for (int p0 = first; p0 < total; p0 += step, buf ^= 1) {
             const int m = min(KTILE, total - p0);
-            if (p0 + KTILE < total) stage(p0 + KTILE, buf ^ 1);
+            if (p0 + step < total) stage(p0 + step, buf ^ 1);
             cp_async_commit();
             cp_async_wait_prev();  // this thread's copies into tile[buf] have landed
             __syncthreads();       // ... and every other thread's
@@ -2067,6 +2174,10 @@ __device__ __forceinline__ void near_batch(const NearArgs& A, int64_t b) {
             }
             __syncthreads();  // tile[buf] is read before the next stage refills it
         }
+        if constexpr (kSplit) {  // the chunk's tiles count on: tile i of the batch belongs to block i mod parts
+            const int tiles = (total + KTILE - 1) / KTILE;
+            turn = ((turn - tiles) % cp.parts + cp.parts) % cp.parts;
+        }
     }
     if constexpr (KS > 1) {  // add the other groups' sums to group 0's through the (consumed) tile buffer
         double* red = reinterpret_cast<double*>(&tile[0][0]);
@@ -2077,13 +2188,32 @@ __device__ __forceinline__ void near_batch(const NearArgs& A, int64_t b) {
 #pragma unroll
                 for (int c = 0; c < 3; ++c) red[(((part - 1) * kT + u) * 3 + c) * kTT + tid] = D[u][c];
         __syncthreads();
-        if (part > 0) return;  // block-uniform barriers follow only in next_batch
+        if (!kSplit && part > 0) return;  // block-uniform barriers follow only in next_batch
+        if (part == 0)
 #pragma unroll
-        for (int g = 1; g < KS; ++g)
+            for (int g = 1; g < KS; ++g)
+#pragma unroll
+                for (int u = 0; u < kT; ++u)
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) D[u][c] += red[(((g - 1) * kT + u) * 3 + c) * kTT + tid];
+    }
+    if constexpr (kSplit) {  // block 0 adds the blocks' sums in rank order
+        double* red = reinterpret_cast<double*>(&tile[1][0]);
+        __syncthreads();
+        if (cp.rank > 0 && part == 0)
 #pragma unroll
             for (int u = 0; u < kT; ++u)
 #pragma unroll
-                for (int c = 0; c < 3; ++c) D[u][c] += red[(((g - 1) * kT + u) * 3 + c) * kTT + tid];
+                for (int c = 0; c < 3; ++c) red[(u * 3 + c) * kTT + tid] = D[u][c];
+        cluster_barrier();
+        if (cp.rank == 0 && part == 0)
+            for (int r = 1; r < cp.parts; ++r)
+#pragma unroll
+                for (int u = 0; u < kT; ++u)
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) D[u][c] += cluster_load(red + (u * 3 + c) * kTT + tid, r);
+        cluster_barrier();  // the sums are read before their space is filled again
+        if (cp.rank > 0 || part > 0) return;
     }
 #pragma unroll
     for (int u = 0; u < kT; ++u) {
@@ -2105,15 +2235,32 @@ __global__ void __launch_bounds__(kBatch / KT * KS) near_kernel(NearArgs A) {
         near_batch<kScalar, KT, KTILE, KS>(A, b);
 }
 
+template <bool kScalar, int KT, int KTILE, int KS>
+__global__ void __launch_bounds__(kBatch / KT * KS) near_split_kernel(NearArgs A, int parts) {
+    __shared__ int32_t slot[2];
+    const ClusterPart cp{(int)(blockIdx.x % (unsigned)parts), parts};
+    const int nbat = *A.nbat;
+    cluster_barrier();  // every block of the cluster runs before another touches its shared memory
+    for (int round = 0;; ++round) {
+        const int64_t b = next_batch_split(A.ticket, A.order, nbat, slot, round, cp);
+        if (b < 0) break;
+        near_batch<kScalar, KT, KTILE, KS, true>(A, b, cp);
+    }
+}
+
 typedef void (*NearFn)(NearArgs);
+typedef void (*NearSplitFn)(NearArgs, int);
 
 // The near kernel of a tile shape (targets per thread 2 or 4; staged sources 256, 512 or 1024; 1 or 2
-// source groups) and its block size; nullptr for another shape.
-NearFn near_select(bool scalar, int targets, int tile, int split, int* threads) {
+// source groups), its block size and its cluster launch; nullptr for another shape.
+NearFn near_select(bool scalar, int targets, int tile, int split, int* threads, NearSplitFn* cluster = nullptr) {
     *threads = kBatch / targets * split;
 #define LPM_NEAR_CASE(T, TILE, S)                                     \
-    if (targets == T && tile == TILE && split == S)                    \
-        return scalar ? near_kernel<true, T, TILE, S> : near_kernel<false, T, TILE, S>;
+    if (targets == T && tile == TILE && split == S) {                  \
+        if (cluster)                                                   \
+            *cluster = scalar ? near_split_kernel<true, T, TILE, S> : near_split_kernel<false, T, TILE, S>; \
+        return scalar ? near_kernel<true, T, TILE, S> : near_kernel<false, T, TILE, S>;                     \
+    }
     LPM_NEAR_CASE(2, 256, 1)
     LPM_NEAR_CASE(2, 512, 1)
     LPM_NEAR_CASE(2, 1024, 1)
@@ -2404,7 +2551,8 @@ struct TreeSolver {
     uint32_t* far_work = nullptr;     // per batch: far coefficient evaluations (count pass)
     int32_t* sched_order = nullptr;   // batches by decreasing near work
     int32_t* far_order = nullptr;     // batches by decreasing far work
-    int near_blocks = 1;              // persistent grids: resident blocks on the whole device
+    int near_blocks = 1;              // persistent grids: resident blocks on the whole device, at most the batch capacity
+    int near_resident = 1;            // the same without that bound
     int near_targets = kNearTargets;  // near kernel tile shape (run-time "near_targets", "near_tile")
     int near_tile = kNearStreamTile;
     int near_split = kNearSplit;      // source groups per batch (run-time "near_split")
@@ -2413,6 +2561,7 @@ struct TreeSolver {
     int far_low_blocks = 1;             // far_low2_kernel (FP32 orders 1..kFarLowMax in one launch)
     uint64_t generation = 0;          // reallocations of the lists and per-node arrays (tree_generation)
     int32_t* state = nullptr;         // pinned host copy of the zero block (read_state)
+    bool clusters = true;             // few batches may run as clusters (cluster_parts)
     bool sized = false;               // an uncaptured evaluation has succeeded: the buffers fit such inputs
     std::vector<void*> allocs;
 };
@@ -2518,6 +2667,7 @@ static int near_shape(TreeSolver* t, int targets, int tile, int split) {
     t->near_targets = targets;
     t->near_tile = tile;
     t->near_split = split;
+    t->near_resident = std::max(per_sm, 1) * t->ctx->num_sms;
     t->near_blocks = (int)std::max<int64_t>(1, std::min<int64_t>(t->n_batches,
                                                                   (int64_t)std::max(per_sm, 1) * t->ctx->num_sms));
     return LPM_OK;
@@ -2736,7 +2886,7 @@ int tree_solver_create(lpm_ctx* ctx, const lpm_kernel_desc& kernel, const lpm_so
                 int threads = 0;
                 per_sm = 0;
                 if (scalar) {
-                    FarScalarFn fs = far_scalar_select(P, f64 != 0, &smem, &threads);
+                    FarScalarFn fs = far_scalar_select(P, f64 != 0, false, &smem, &threads);
                     ea = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fs, threads, smem);
                 } else {
                     FarKernelFn fn = far_kernel_select(P, f64 != 0, &smem, &threads);
@@ -3050,7 +3200,32 @@ static NearArgs near_args(const TreeSolver* t, double* U) {
 }
 
 // Order P's far-field launch(es) of t on its context's stream, on the schedule tree_prepare made.
-static int tree_far_order(TreeSolver* t, int P) {
+// Blocks per batch of the far and near launches, by the batches there are for each SM (about 110 targets each).  A batch
+// is a chain of stages; with few batches the longest chains decide, and a cluster shortens them, for three cluster
+// barriers a batch.  Measured, us per evaluation with 1 / 2 / 4 blocks a batch in both launches: fixed order 8 on 15,000
+// / 37,500 / 75,000 / 123,000 / 240,000 targets 446 / 355 / 311, 666 / 472 / 413, 882 / 572 / 568, 851 / 793 / 830,
+// 1340 / 1320 / 1456; learned orders (a few clusters per order and batch: the far launches gain less) on 15,000 / 37,500 /
+// 123,000 647 / 540 / 505, 1047 / 771 / 723, 1379 / 1352 / 1516; Poisson on 10,000 / 25,000 / 50,000 / 100,000 points
+// 339 / 277 / 253, 458 / 371 / 359, 471 / 425 / 447, 671 / 665 / 714, its far launch alone in two parts 1279 -> 1223 at
+// 200,000.
+struct ClusterParts {
+    int far, near;
+};
+static ClusterParts cluster_parts(const TreeSolver* t) {
+    if (!t->clusters) return ClusterParts{1, 1};
+    const double per_sm = (double)t->n_tgt / 110.0 / std::max(t->ctx->num_sms, 1);
+    auto rule = [&](double four, double two) { return per_sm <= four ? 4 : (per_sm <= two ? 2 : 1); };
+    if (t->scalar) return ClusterParts{rule(1.7, 14.0), rule(2.4, 6.0)};
+    const bool learned = t->learned && t->mlp_loaded;
+    return ClusterParts{learned ? rule(0.0, 2.8) : rule(2.8, 8.5), rule(2.4, 9.0)};
+}
+
+// A persistent grid of `blocks` resident blocks as whole clusters of `parts`.
+static unsigned cluster_grid(unsigned blocks, int parts) {
+    return std::max(1u, blocks / (unsigned)parts) * (unsigned)parts;
+}
+
+static int tree_far_order(TreeSolver* t, int P, int parts) {
     lpm_ctx* ctx = t->ctx;
     FarArgs F = far_args(t, P);
     size_t smem = 0;
@@ -3060,19 +3235,31 @@ static int tree_far_order(TreeSolver* t, int P) {
         F.B64 = (const double4*)t->A64;
         F.B32 = (const float4*)t->A32;
         int threads = 0;
-        FarScalarFn fs = far_scalar_select(P, f64, &smem, &threads);
-        LPM_LAUNCH(ctx, "far_kernel", fs, grid, threads, smem, F, t->a_stride);
+        if (f64 || P > kFar2ScalarMaxOrder) parts = 1;
+        FarScalarFn fs = far_scalar_select(P, f64, parts > 1, &smem, &threads);
+        return launch_cluster(ctx, "far_kernel", fs, cluster_grid(grid, parts), threads, smem, parts, F, t->a_stride,
+                              parts);
     } else if (P == kFarSplitOrder && !f64) {  // two launches, each on its own ticket
         for (int part = 1; part <= 2; ++part) {
             int threads = 0;
             FarKernelFn fn = far_split_select(part, &smem, &threads);
             F.gtab = t->gtab + t->ct.table_off[P] + (part == 2 ? part_entries(P, 1) : 0);
             F.ticket = t->zero + kZeroFarTicket + (part == 2 ? kPMax + 1 : P);
-            LPM_LAUNCH(ctx, "far_kernel", fn, (unsigned)t->far_split_blocks[part - 1], threads, smem, F);
+            const unsigned g = (unsigned)t->far_split_blocks[part - 1];
+            if (parts > 1) {
+                const int rc = launch_cluster(ctx, "far_kernel", far_cluster_select(P, part), cluster_grid(g, parts),
+                                              threads, smem, parts, F, parts);
+                if (rc) return rc;
+            } else {
+                LPM_LAUNCH(ctx, "far_kernel", fn, g, threads, smem, F);
+            }
         }
     } else {
         int threads = 0;
         FarKernelFn fn = far_kernel_select(P, f64, &smem, &threads);
+        if (parts > 1 && !f64 && P <= kFar2MaxOrder)
+            return launch_cluster(ctx, "far_kernel", far_cluster_select(P, 0), cluster_grid(grid, parts), threads, smem,
+                                  parts, F, parts);
         LPM_LAUNCH(ctx, "far_kernel", fn, grid, threads, smem, F);
     }
     return LPM_OK;
@@ -3089,6 +3276,8 @@ static int tree_enqueue(TreeSolver* t, const double4* src, int64_t n_src, const 
     int rc = tree_prepare(t, src, n_src, X, n_tgt, U, true, careful, &pending);
     if (rc || !pending) return rc;
     const unsigned gt = (unsigned)std::max<int64_t>(1, std::min<int64_t>(grid_for(n_tgt + 1, 256), 8 * ctx->num_sms));
+    const ClusterParts parts = cluster_parts(t);
+    const int far_parts = parts.far, near_parts = parts.near;
     // near field: batches by decreasing near work, taken by a persistent grid.  Biot-Savart: after the far
     // field on the context's stream, writing u = mult (V - x cross D).  Scalar kernel: it writes W only and runs
     // on the solver's side stream beside the far-field launch, filling its tail (1M Poisson points: 7.37 ->
@@ -3098,7 +3287,11 @@ static int tree_enqueue(TreeSolver* t, const double4* src, int64_t n_src, const 
     auto launch_near = [&]() -> int {
         const NearArgs N = near_args(t, U);
         int threads = 0;
-        NearFn fn = near_select(t->scalar, t->near_targets, t->near_tile, t->near_split, &threads);
+        NearSplitFn split = nullptr;
+        NearFn fn = near_select(t->scalar, t->near_targets, t->near_tile, t->near_split, &threads, &split);
+        if (near_parts > 1)
+            return launch_cluster(ctx, "near_kernel", split, cluster_grid((unsigned)t->near_resident, near_parts), threads,
+                                  (size_t)0, near_parts, N, near_parts);
         LPM_LAUNCH(ctx, "near_kernel", fn, (unsigned)t->near_blocks, threads, 0, N);
         return LPM_OK;
     };
@@ -3110,12 +3303,19 @@ static int tree_enqueue(TreeSolver* t, const double4* src, int64_t n_src, const 
     if (!t->scalar && low_hi > p_lo && low_hi < t->f64_from) {  // FP32 orders p_lo..low_hi in one launch
         FarLowArgs LA{};
         for (int P = p_lo; P <= low_hi; ++P) LA.a[P - 1] = far_args(t, P);
-        LPM_LAUNCH(ctx, "far_kernel", far_low2_kernel, (unsigned)t->far_low_blocks, kFar2Threads, far_low_smem(), LA,
-                   t->tcount + 1, t->far_order, t->zero + kZeroFarTicket + p_lo);
+        if (far_parts > 1) {
+            rc = launch_cluster(ctx, "far_kernel", far_low2_split_kernel, cluster_grid((unsigned)t->far_low_blocks, far_parts),
+                                kFar2Threads, far_low_smem(), far_parts, LA, t->tcount + 1, t->far_order,
+                                t->zero + kZeroFarTicket + p_lo, far_parts);
+            if (rc) return rc;
+        } else {
+            LPM_LAUNCH(ctx, "far_kernel", far_low2_kernel, (unsigned)t->far_low_blocks, kFar2Threads, far_low_smem(), LA,
+                       t->tcount + 1, t->far_order, t->zero + kZeroFarTicket + p_lo);
+        }
         p_lo = low_hi + 1;
     }
     for (int P = p_lo; P <= p_hi; ++P) {
-        rc = tree_far_order(t, P);
+        rc = tree_far_order(t, P, far_parts);
         if (rc) return rc;
     }
     if (overlap) {  // enqueued after the far launches: the near blocks fill the SMs as far blocks retire
@@ -3348,7 +3548,7 @@ int tree_fused_run(TreeFused* f) {
             TreeSolver* t = f->ts[sp.first];
             cudaStream_t own = t->ctx->stream;
             t->ctx->stream = ctx->stream;
-            const int rc = tree_far_order(t, P);
+            const int rc = tree_far_order(t, P, 1);
             t->ctx->stream = own;
             if (rc) return rc;
         }
@@ -3407,6 +3607,8 @@ int tree_check(TreeSolver* t) {
 }
 
 uint64_t tree_generation(const TreeSolver* t) { return t->generation; }
+
+void tree_set_clusters(TreeSolver* t, bool on) { t->clusters = on; }
 
 const Octree& tree_source_octree(const TreeSolver* t, int64_t* n_points) {
     *n_points = t->n_src;

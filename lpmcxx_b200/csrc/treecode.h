@@ -40,6 +40,10 @@ int tree_fused_bind(TreeFused* f, TreeSolver* const* ts, double* const* Us, int 
 int tree_fused_run(TreeFused* f);
 // Synchronises and reports capacity overflows of the last evaluation (LPM_ERR_CAPACITY).
 int tree_check(TreeSolver* t);
+// Whether evaluations of few batches may run each batch on a cluster of blocks (default on).  Off for an ensemble's
+// instances: they fill the device together, and every batch is then summed by one block in the fused launches and in
+// the instances' own ones alike (the same FP64 order of additions).
+void tree_set_clusters(TreeSolver* t, bool on);
 // nodes, leaves, depth, far (batch, cluster) pairs, near runs, batches, overflow flags,
 // far target-cluster evaluations, near target-source pairs, far coefficient evaluations (sum over far
 // evaluations of the order's coefficient count) (10 values; synchronises)
