@@ -1074,6 +1074,7 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
 }
 
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_prev() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
 
 template <typename F, typename F4>
@@ -1222,7 +1223,7 @@ __device__ __forceinline__ void horner2_f32x2(const float4* __restrict__ Bc, con
     int q = 0;
     float G[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
 #pragma unroll
-    for (int m = PART == 2 ? 0 : (P - 1) / 2; m >= (PART == 1 ? 1 : 0); --m) {
+    for (int m = PART == 2 ? 0 : (P - 1) / 2; m >= 0; --m) {
         const int Q = P - 2 * m;
         float Pa[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
 #pragma unroll
@@ -1274,10 +1275,6 @@ __device__ __forceinline__ void horner2_f32x2(const float4* __restrict__ Bc, con
             }
         }
     }
-    if constexpr (PART == 1) {  // the blocks m >= 1 carry one more factor s
-#pragma unroll
-        for (int c = 0; c < 4; ++c) fma2v(G[0][c], G[1][c], G[0][c], G[1][c], e[0][3], e[1][3], -0.0f, -0.0f);
-    }
 #pragma unroll
     for (int t = 0; t < 2; ++t)
 #pragma unroll
@@ -1319,7 +1316,16 @@ __device__ __forceinline__ void far_one_acc2_f32(const float4* __restrict__ Bc, 
     e[1][3] = rcp32(r1);
 #pragma unroll
     for (int k = 0; k < 3; ++k) fma2v(e[0][k], e[1][k], d[0][k], d[1][k], e[0][3], e[1][3], -0.0f, -0.0f);
-    horner2_f32x2<P, PART>(Bc, e, g);
+    if constexpr (PART == 1) {  // the blocks m >= 1: the sequence of order P - 2, with one more factor s
+        horner2_f32x2<P - 2>(Bc, e, g);
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {  // packed as the scheme leaves them, component by component
+            fma2p(g[t][0], g[t][1], g[t][0], g[t][1], e[t][3], -0.0f, -0.0f);
+            fma2p(g[t][2], g[t][3], g[t][2], g[t][3], e[t][3], -0.0f, -0.0f);
+        }
+    } else {
+        horner2_f32x2<P, PART>(Bc, e, g);
+    }
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         float h0, h1;
@@ -1328,32 +1334,51 @@ __device__ __forceinline__ void far_one_acc2_f32(const float4* __restrict__ Bc, 
     }
 }
 
-// Stage gather of the far2 kernel: coefficients by cp.async as far_stage_gather, cluster centres as FP32
-// offsets from the block's origin o.
+// Shared memory of the far2 kernel: two stages of kK entries' coefficients, then for a chunk of kChunk entries of the
+// batch's list their centres (FP32 offsets) and node indices, then the gather table (entry of the stage and canonical
+// index of every unit).
+constexpr int kFarChunkMax = 128;
 template <int P, int PART = 0>
-__device__ __forceinline__ void far2_stage_gather(const FarArgs& A, int64_t s0, int n, float4* buf, float4* ctr,
-                                                  const double4& o) {
-    constexpr int kUnits = FarShape<P, float4, kFarStageUnits, PART>::kUnits;
-    for (int i = threadIdx.x; i < n * kUnits; i += kFar2Threads) {
-        const int e = i / kUnits, j = i - e * kUnits;
-        const int node = A.far_list[s0 + e].x;
-        cp_async16(buf + i, A.B32 + (size_t)node * A.n_ent + A.gtab[j]);
-    }
-    if ((int)threadIdx.x < n) {
-        const double4 c = A.node_ctr[A.far_list[s0 + threadIdx.x].x];
-        ctr[threadIdx.x] = make_float4((float)(c.x - o.x), (float)(c.y - o.y), (float)(c.z - o.z), 0.0f);
+struct Far2Shape {
+    using S = FarShape<P, float4, kFar2StageUnits, PART>;
+    static constexpr int kK = S::kK, kUnits = S::kUnits, kStage = S::kStage;
+    static constexpr int kChunkStages = kFarChunkMax / kK, kChunk = kChunkStages * kK;
+    static constexpr size_t kSmem = sizeof(float4) * (2 * kStage + kChunk) + sizeof(int32_t) * kChunk +
+                                    sizeof(uint16_t) * ((kStage + 1) & ~1);
+    static_assert(sizeof(float4) * (2 * kStage + kChunk) >= 6 * kFar2Threads * sizeof(double), "a split batch's sums fit");
+};
+constexpr int kFarTabShift = 10;  // canonical indices are below 1024 (kPMax: 728 entries), entries of a stage below 64
+static_assert(entries_for(kPMax) < (1 << kFarTabShift), "gather table packing");
+
+// The gather table's place, and the table of order P (part PART) from the solver's canonical indices, written by the
+// whole block; the chunk loop's barriers order it before its readers.
+template <int P, int PART = 0>
+__device__ __forceinline__ uint16_t* far2_tab(float4* fbuf) {
+    using S = Far2Shape<P, PART>;
+    return reinterpret_cast<uint16_t*>(reinterpret_cast<int32_t*>(fbuf + 2 * S::kStage + S::kChunk) + S::kChunk);
+}
+template <int P, int PART = 0>
+__device__ __forceinline__ void far2_table(const int32_t* __restrict__ gtab, uint16_t* tab) {
+    using S = Far2Shape<P, PART>;
+    for (int i = threadIdx.x; i < S::kStage; i += kFar2Threads) {
+        const int e = i / S::kUnits;
+        tab[i] = (uint16_t)((e << kFarTabShift) | gtab[i - e * S::kUnits]);
     }
 }
 
-// One batch b of the far2 kernel (the whole block); fbuf: 2 stages of S::kStage units, then 2 x kK centres
-// (FP32 offsets).
+// One batch b of the far2 kernel (the whole block).  The list's node indices and centres come a chunk at a time into
+// shared memory, so that a stage's gather reads no global memory before its copies: with the indices read per unit and
+// the centres per stage, every stage began with two dependent round trips, and the kernel ran at 2.90 cycles per packed
+// FMA (order 8) where its arithmetic alone takes 2.43.  A stage is one barrier: the next one's copies go to the buffer
+// whose readers that barrier has collected.
 template <int P, int PART = 0, bool kSplit = false>
-__device__ __forceinline__ void far2_batch(const FarArgs& A, int64_t b, float4* fbuf, ClusterPart cp = {0, 1}) {
-    using S = FarShape<P, float4, kFar2StageUnits, PART>;
+__device__ __forceinline__ void far2_batch(const FarArgs& A, int64_t b, float4* fbuf, const uint16_t* tab,
+                                           ClusterPart cp = {0, 1}) {
+    using S = Far2Shape<P, PART>;
     float4* ctr = fbuf + 2 * S::kStage;
+    int32_t* ids = reinterpret_cast<int32_t*>(ctr + S::kChunk);
     const int64_t f0 = A.far_off[b], f1 = min(f0 + (int64_t)A.far_cnt[b], A.far_cap);
     if (f0 >= f1) return;  // uniform per block (and cluster)
-    const int64_t step = kSplit ? (int64_t)S::kK * cp.parts : S::kK, first = kSplit ? f0 + (int64_t)S::kK * cp.rank : f0;
     const int64_t q0 = A.batch_first[b], qe = A.batch_first[b + 1];
     // warp w holds targets 64 w .. 64 w + 63 of the batch (lane l: 64 w + l and 64 w + l + 32), so a warp past
     // the batch's last target idles as a whole (batches average ~109 of 128 targets)
@@ -1368,32 +1393,50 @@ __device__ __forceinline__ void far2_batch(const FarArgs& A, int64_t b, float4* 
         xo[t][0] = (float)(p.x - o.x); xo[t][1] = (float)(p.y - o.y); xo[t][2] = (float)(p.z - o.z);
     }
     double acc[2][3] = {{0, 0, 0}, {0, 0, 0}};
-    if (!kSplit || first < f1) far2_stage_gather<P, PART>(A, first, (int)min((int64_t)S::kK, f1 - first), fbuf, ctr, o);
-    cp_async_commit();
-    int s = 0;
-    for (int64_t s0 = first; !kSplit || s0 < f1; s ^= 1) {
-        const int n = (int)min((int64_t)S::kK, f1 - s0);
-        const int64_t s1 = kSplit ? s0 + step : s0 + n;
-        if (s1 < f1)
-            far2_stage_gather<P, PART>(A, s1, (int)min((int64_t)S::kK, f1 - s1), fbuf + (size_t)(s ^ 1) * S::kStage,
-                                 ctr + (s ^ 1) * S::kK, o);
-        cp_async_commit();
-        cp_async_wait_prev();
-        __syncthreads();  // stage s resident
-        if (live) {
-            const float4* Bc = fbuf + (size_t)s * S::kStage;
-            const float4* cs = ctr + s * S::kK;
-            float acc32[2][3] = {{0, 0, 0}, {0, 0, 0}};
-            for (int k = 0; k < n; ++k)
-                far_one_acc2_f32<P, PART>(Bc + (size_t)k * part_entries(P, PART), xo, cs[k], acc32);
-#pragma unroll
-            for (int t = 0; t < 2; ++t)
-#pragma unroll
-                for (int c = 0; c < 3; ++c) acc[t][c] += (double)acc32[t][c];
+    int s = 0, turn = cp.rank;  // split: stages until this block's next one
+    for (int64_t c0 = f0; c0 < f1; c0 += S::kChunk) {
+        const int cn = (int)min((int64_t)S::kChunk, f1 - c0);
+        __syncthreads();  // the previous chunk's (batch's, order's) readers are done
+        for (int i = threadIdx.x; i < cn; i += kFar2Threads) {
+            const int node = A.far_list[c0 + i].x;
+            ids[i] = node;
+            const double4 c = A.node_ctr[node];
+            ctr[i] = make_float4((float)(c.x - o.x), (float)(c.y - o.y), (float)(c.z - o.z), 0.0f);
         }
-        if (s1 >= f1) break;
-        __syncthreads();  // stage s consumed before it is refilled
-        s0 = s1;
+        __syncthreads();
+        auto gather = [&](int st, float4* to) {  // the coefficients of stage st of the chunk
+            const int n = min(S::kK, cn - st * S::kK) * S::kUnits;
+            for (int i = threadIdx.x; i < n; i += kFar2Threads) {
+                const int t = tab[i];
+                const int node = ids[st * S::kK + (t >> kFarTabShift)];
+                cp_async16(to + i, A.B32 + (size_t)node * A.n_ent + (t & ((1 << kFarTabShift) - 1)));
+            }
+        };
+        const int step = kSplit ? cp.parts : 1;
+        int st = kSplit ? turn : 0;
+        if (st * S::kK < cn) gather(st, fbuf + (size_t)s * S::kStage);
+        for (; st * S::kK < cn; st += step, s ^= 1) {
+            cp_async_wait_all();
+            __syncthreads();  // stage s has landed; the other buffer's readers are done
+            if ((st + step) * S::kK < cn) gather(st + step, fbuf + (size_t)(s ^ 1) * S::kStage);
+            if (live) {
+                const int n = min(S::kK, cn - st * S::kK);
+                const float4* Bc = fbuf + (size_t)s * S::kStage;
+                const float4* cs = ctr + st * S::kK;
+                float acc32[2][3] = {{0, 0, 0}, {0, 0, 0}};
+#pragma unroll 1
+                for (int k = 0; k < n; ++k)
+                    far_one_acc2_f32<P, PART>(Bc + (size_t)k * part_entries(P, PART), xo, cs[k], acc32);
+#pragma unroll
+                for (int t = 0; t < 2; ++t)
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) acc[t][c] += (double)acc32[t][c];
+            }
+        }
+        if constexpr (kSplit) {  // the chunk's stages count on: stage i of the batch belongs to block i mod parts
+            const int stages = (cn + S::kK - 1) / S::kK;
+            turn = ((turn - stages) % cp.parts + cp.parts) % cp.parts;
+        }
     }
     if constexpr (kSplit) {  // block 0 adds the blocks' sums in rank order
         double* red = reinterpret_cast<double*>(fbuf);
@@ -1436,8 +1479,9 @@ __global__ void __launch_bounds__(kFar2Threads, kFar2MinBlocks) far_order2_kerne
     extern __shared__ float4 fbuf[];
     __shared__ int slot;
     const int nbat = *A.nbat;
+    far2_table<P, PART>(A.gtab, far2_tab<P, PART>(fbuf));
     for (int64_t b = next_batch(A.ticket, A.order, nbat, &slot); b >= 0; b = next_batch(A.ticket, A.order, nbat, &slot))
-        far2_batch<P, PART>(A, b, fbuf);
+        far2_batch<P, PART>(A, b, fbuf, far2_tab<P, PART>(fbuf));
 }
 
 template <int P, int PART = 0>
@@ -1446,11 +1490,12 @@ __global__ void __launch_bounds__(kFar2Threads, kFar2MinBlocks) far_order2_split
     __shared__ int32_t slot[2];
     const ClusterPart cp{(int)(blockIdx.x % (unsigned)parts), parts};
     const int nbat = *A.nbat;
+    far2_table<P, PART>(A.gtab, far2_tab<P, PART>(fbuf));
     cluster_barrier();  // every block of the cluster runs before another touches its shared memory
     for (int round = 0;; ++round) {
         const int64_t b = next_batch_split(A.ticket, A.order, nbat, slot, round, cp);
         if (b < 0) break;
-        far2_batch<P, PART, true>(A, b, fbuf, cp);
+        far2_batch<P, PART, true>(A, b, fbuf, far2_tab<P, PART>(fbuf), cp);
     }
 }
 
@@ -1463,23 +1508,41 @@ struct FarLowArgs {
     FarArgs a[kFarLowMax];  // a[P - 1]: order P's arguments; far_cnt null: order P is not in this launch
 };
 
+// One batch of far_low2_kernel: every order's body in turn, each behind its own gather table.
+template <bool kSplit>
+__device__ __forceinline__ void far_low_batch(const FarLowArgs& L, int64_t b, float4* fbuf, uint16_t* const (&tab)[kFarLowMax],
+                                              ClusterPart cp) {
+    if (L.a[0].far_cnt) far2_batch<1, 0, kSplit>(L.a[0], b, fbuf, tab[0], cp);
+    if (L.a[1].far_cnt) far2_batch<2, 0, kSplit>(L.a[1], b, fbuf, tab[1], cp);
+    if (L.a[2].far_cnt) far2_batch<3, 0, kSplit>(L.a[2], b, fbuf, tab[2], cp);
+    if (L.a[3].far_cnt) far2_batch<4, 0, kSplit>(L.a[3], b, fbuf, tab[3], cp);
+}
+// The gather tables of orders 1..4, back to back.
+constexpr int kFarLowTab = Far2Shape<1>::kStage + Far2Shape<2>::kStage + Far2Shape<3>::kStage + Far2Shape<4>::kStage;
+__device__ __forceinline__ void far_low_tables(const FarLowArgs& L, uint16_t* space, uint16_t* (&tab)[kFarLowMax]) {
+    static_assert(kFarLowMax == 4 && kFarLowMax < kFarSplitOrder, "orders 1..4, none split");
+    tab[0] = space;
+    tab[1] = tab[0] + Far2Shape<1>::kStage;
+    tab[2] = tab[1] + Far2Shape<2>::kStage;
+    tab[3] = tab[2] + Far2Shape<3>::kStage;
+    if (L.a[0].far_cnt) far2_table<1>(L.a[0].gtab, tab[0]);
+    if (L.a[1].far_cnt) far2_table<2>(L.a[1].gtab, tab[1]);
+    if (L.a[2].far_cnt) far2_table<3>(L.a[2].gtab, tab[2]);
+    if (L.a[3].far_cnt) far2_table<4>(L.a[3].gtab, tab[3]);
+}
+
 __global__ void __launch_bounds__(kFar2Threads, kFar2MinBlocks) far_low2_kernel(FarLowArgs L,
                                                                                const int32_t* __restrict__ nbat_p,
                                                                                const int32_t* __restrict__ order,
                                                                                int32_t* ticket) {
-    static_assert(kFarLowMax == 4 && kFarLowMax < kFarSplitOrder, "orders 1..4, none split");
     extern __shared__ float4 fbuf[];
+    __shared__ uint16_t space[kFarLowTab];
     __shared__ int slot;
     const int nbat = *nbat_p;
-    for (int64_t b = next_batch(ticket, order, nbat, &slot); b >= 0; b = next_batch(ticket, order, nbat, &slot)) {
-        if (L.a[0].far_cnt) far2_batch<1>(L.a[0], b, fbuf);
-        __syncthreads();  // the previous order's stage buffers are read before the next order's gathers
-        if (L.a[1].far_cnt) far2_batch<2>(L.a[1], b, fbuf);
-        __syncthreads();
-        if (L.a[2].far_cnt) far2_batch<3>(L.a[2], b, fbuf);
-        __syncthreads();
-        if (L.a[3].far_cnt) far2_batch<4>(L.a[3], b, fbuf);
-    }
+    uint16_t* tab[kFarLowMax];
+    far_low_tables(L, space, tab);
+    for (int64_t b = next_batch(ticket, order, nbat, &slot); b >= 0; b = next_batch(ticket, order, nbat, &slot))
+        far_low_batch<false>(L, b, fbuf, tab, ClusterPart{0, 1});
 }
 
 __global__ void __launch_bounds__(kFar2Threads, kFar2MinBlocks) far_low2_split_kernel(FarLowArgs L,
@@ -1487,24 +1550,23 @@ __global__ void __launch_bounds__(kFar2Threads, kFar2MinBlocks) far_low2_split_k
                                                                                      const int32_t* __restrict__ order,
                                                                                      int32_t* ticket, int parts) {
     extern __shared__ float4 fbuf[];
+    __shared__ uint16_t space[kFarLowTab];
     __shared__ int32_t slot[2];
     const ClusterPart cp{(int)(blockIdx.x % (unsigned)parts), parts};
     const int nbat = *nbat_p;
+    uint16_t* tab[kFarLowMax];
+    far_low_tables(L, space, tab);
     cluster_barrier();  // every block of the cluster runs before another touches its shared memory
     for (int round = 0;; ++round) {  // every far2_batch with work ends in a cluster barrier
         const int64_t b = next_batch_split(ticket, order, nbat, slot, round, cp);
         if (b < 0) break;
-        if (L.a[0].far_cnt) far2_batch<1, 0, true>(L.a[0], b, fbuf, cp);
-        if (L.a[1].far_cnt) far2_batch<2, 0, true>(L.a[1], b, fbuf, cp);
-        if (L.a[2].far_cnt) far2_batch<3, 0, true>(L.a[2], b, fbuf, cp);
-        if (L.a[3].far_cnt) far2_batch<4, 0, true>(L.a[3], b, fbuf, cp);
+        far_low_batch<true>(L, b, fbuf, tab, cp);
     }
 }
 
-// Dynamic shared memory of far_low2_kernel: the largest of its orders' stage buffers.
+// Dynamic shared memory of far_low2_kernel: the largest of its orders' buffers.
 size_t far_low_smem() {
-    return std::max(std::max(FarShape<1, float4, kFar2StageUnits>::kSmem, FarShape<2, float4, kFar2StageUnits>::kSmem),
-                    std::max(FarShape<3, float4, kFar2StageUnits>::kSmem, FarShape<4, float4, kFar2StageUnits>::kSmem));
+    return std::max(std::max(Far2Shape<1>::kSmem, Far2Shape<2>::kSmem), std::max(Far2Shape<3>::kSmem, Far2Shape<4>::kSmem));
 }
 
 // The Horner scheme of `horner` with scalar coefficients.
@@ -1774,7 +1836,7 @@ FarKernelFn far_kernel_for(bool f64, size_t* smem, int* threads) {
     }
     if constexpr (P <= kFar2MaxOrder) {
         *threads = kFar2Threads;
-        *smem = FarShape<P, float4, kFar2StageUnits>::kSmem;
+        *smem = Far2Shape<P>::kSmem;
         return far_order2_kernel<P>;
     }
     *smem = FarShape<P, float4>::kSmem;
@@ -1806,10 +1868,10 @@ FarSplitFn far_cluster_select(int P, int part) {
 FarKernelFn far_split_select(int part, size_t* smem, int* threads) {
     *threads = kFar2Threads;
     if (part == 1) {
-        *smem = FarShape<kFarSplitOrder, float4, kFar2StageUnits, 1>::kSmem;
+        *smem = Far2Shape<kFarSplitOrder, 1>::kSmem;
         return far_order2_kernel<kFarSplitOrder, 1>;
     }
-    *smem = FarShape<kFarSplitOrder, float4, kFar2StageUnits, 2>::kSmem;
+    *smem = Far2Shape<kFarSplitOrder, 2>::kSmem;
     return far_order2_kernel<kFarSplitOrder, 2>;
 }
 
@@ -2379,7 +2441,16 @@ __global__ void __launch_bounds__(kFar2Threads, kFar2MinBlocks) far_fused2_kerne
     __shared__ int2 item;
     const FarArgs& A = *reinterpret_cast<const FarArgs*>(araw);
     const int n = *S.total;
-    while (next_fused_item(S, n, tab, araw, &item)) far2_batch<P, PART>(A, item.y, fbuf);
+    __shared__ const int32_t* gtab;  // the gather table follows the item's solver
+    if (threadIdx.x == 0) gtab = nullptr;
+    while (next_fused_item(S, n, tab, araw, &item)) {
+        if (A.gtab != gtab) {  // uniform per block
+            __syncthreads();
+            if (threadIdx.x == 0) gtab = A.gtab;
+            far2_table<P, PART>(A.gtab, far2_tab<P, PART>(fbuf));
+        }
+        far2_batch<P, PART>(A, item.y, fbuf, far2_tab<P, PART>(fbuf));
+    }
 }
 
 // near_kernel (Biot-Savart) over the items of many solvers sharing one tile shape.
@@ -2401,13 +2472,13 @@ template <int P>
 FarFusedFn far_fused_for(int part, size_t* smem) {
     if constexpr (P == kFarSplitOrder) {
         if (part == 2) {
-            *smem = FarShape<P, float4, kFar2StageUnits, 2>::kSmem;
+            *smem = Far2Shape<P, 2>::kSmem;
             return far_fused2_kernel<P, 2>;
         }
-        *smem = FarShape<P, float4, kFar2StageUnits, 1>::kSmem;
+        *smem = Far2Shape<P, 1>::kSmem;
         return far_fused2_kernel<P, 1>;
     } else {
-        *smem = FarShape<P, float4, kFar2StageUnits>::kSmem;
+        *smem = Far2Shape<P>::kSmem;
         return far_fused2_kernel<P>;
     }
 }
