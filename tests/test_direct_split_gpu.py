@@ -101,3 +101,36 @@ def test_values_that_are_not_finite(ctx):
     assert np.isnan(got[:, 7]).all() and np.isfinite(np.delete(got, 7, axis=1)).all()
     phi = _sum(ctx, L.poisson_kernel(), L.LPM_PREC_F64, src, tgt, 1, 0)[0]
     assert rel_linf(phi, oracle.poisson_direct(np.delete(src, 400, axis=0), tgt)) < 1e-12
+
+
+@pytest.mark.parametrize("kernel", [L.sphere_greens_kernel(), L.planar_log_kernel()])
+@pytest.mark.parametrize("scale", [1.0, 3e-60, 7e70])
+def test_log_kernels_to_the_last_bits(ctx, kernel, scale):
+    """One pair per target (the other sources have strength 0), arguments of the logarithm from 2^-9 to 2 (sphere) and
+    over many binades and about 1 (plane), against 80-bit logarithms: 2 units of the last place of the logarithm's two
+    summands (k log 2 and the rest, each below |log| + 0.7), and the sphere's fused argument 3 2^-53 / z."""
+    sphere = kernel.kind == L.sphere_greens_kernel().kind
+    if sphere and scale != 1.0:
+        pytest.skip("the sphere kernel's points have its radius")
+    ctx.use_torch_stream()
+    n = 6001
+    if sphere:
+        t = np.linspace(0.07, np.pi, n)
+        tgt = oracle.pack4(np.stack([np.cos(t), np.sin(t), np.zeros(n)], axis=1))
+    else:
+        r = np.concatenate([np.exp(np.linspace(-12, 12, n - 2001)), 1.0 + np.linspace(-0.02, 0.02, 2001)])
+        tgt = oracle.pack4(np.stack([1.0 + r, np.zeros(n), np.zeros(n)], axis=1) * scale)
+    src = oracle.pack4(np.tile([0.0, 0.0, 1.0], (300, 1)) * scale)
+    src[100] = (scale, 0.0, 0.0, 1.0)
+    got = _sum(ctx, kernel, L.LPM_PREC_F64, src, tgt, 1, 0)[0]
+    x = tgt.astype(np.longdouble)
+    if sphere:
+        z = 1 - x[:, 0]
+        ref, cond = -np.log(z) / (4 * np.longdouble(np.pi)), 3 / z
+    else:
+        d = (x[:, 0] - np.longdouble(src[100, 0]))
+        dr = (tgt[:, 0] - src[100, 0]).astype(np.longdouble)  # x - y rounds once in FP64
+        z, cond = dr * dr, np.abs(2 * (d - dr) / dr) * 2.0 ** 53 + 1
+        ref = np.log(z) / (4 * np.longdouble(np.pi))
+    tol = 2.0 ** -53 * (2 * (2 * np.abs(np.log(z)) + 0.7) + cond) / (4 * np.pi)
+    assert np.max(np.abs(got - ref) / tol) < 1.0
