@@ -404,7 +404,7 @@ struct LogF64 {
 #pragma unroll
         for (int t = 0; t < TPT; ++t) own = own || (self[t] >= j0 && self[t] < j0 + m);
         const bool fast = plain && !__any_sync(0xffffffffu, own);
-#pragma unroll 2
+#pragma unroll 1
         for (int k = 0; k < m; ++k) {
             const double4 y = src[k];
             double z[TPT];
