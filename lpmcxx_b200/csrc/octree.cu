@@ -577,7 +577,8 @@ __device__ __forceinline__ int digit_bound_warp(const uint64_t* __restrict__ key
 // per boundary after), then the child counts' prefix sum (block totals through distributed shared memory) and the
 // children.  Levels stop at the first that splits no node.  Then, level by level again, the leaves below every node
 // are counted upwards and numbered downwards: leaves in depth-first order are numbered by their nodes' order, no
-// pass over the points.  `pending`, if not null, receives every node's number of internal children.
+// pass over the points.  `pending`, if not null, receives every node's number of internal children (-1 for an internal
+// node whose children are all leaves).
 __global__ void __cluster_dims__(kClBlocks, 1, 1) __launch_bounds__(kClThreads)
     tree_nodes_kernel(Octree t, int32_t* __restrict__ pending) {
     __shared__ int32_t slot[2];
@@ -702,7 +703,7 @@ __global__ void __cluster_dims__(kClBlocks, 1, 1) __launch_bounds__(kClThreads)
                 internal += __ldcg(t.node_nchild + fc + k) > 0;
             }
             t.node_leaves[node] = leaves;
-            if (pending) pending[node] = internal;
+            if (pending) pending[node] = nc > 0 && internal == 0 ? -1 : internal;
         }
         cluster_barrier();
     }

@@ -102,7 +102,7 @@ int sort_points(lpm_ctx* ctx, const double4* pts, int64_t n, const RootBox& root
 int octree_alloc(Octree& t, int64_t n, int max_per_leaf, int max_depth, int bits = 3, double sphere_r = 0.0);
 void octree_free(Octree& t);
 // Build over pts[0:n] with the given root box.  Fully asynchronous (capturable): no host reads.  `pending` (node_cap
-// ints, may be null) receives every node's number of internal children.
+// ints, may be null) receives every node's number of internal children, -1 for an internal node of leaves only.
 int octree_build(lpm_ctx* ctx, Octree& t, const double4* pts, int64_t n, const RootBox& root,
                  int32_t* pending = nullptr);
 

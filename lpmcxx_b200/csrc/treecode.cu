@@ -233,11 +233,11 @@ __global__ void __launch_bounds__(kP2mThreads) leaf_p2m_kernel(Octree t, const d
 // Internal nodes: centre = count-weighted mean of the children's centres, radius bound
 // max(|c_child - c| + r_child), moments shifted from the children:
 // m_k(c) = sum_child sum_{j <= k} C(k, j) (c_child - c)^(k-j) m_j(c_child).
-// The children's moments (packed in monomial order), their shift powers and the binomial table are
-// staged in shared memory, so the inner loops read no global or constant memory.
+// The children's moments (packed in monomial order) and the shifts' coefficients are staged in shared memory, so the
+// inner loops read no global or constant memory.
 //
 // One launch does the whole upward pass: pending[node] counts the internal children not yet done; a block
-// starts at each internal node whose children are all leaves (their moments come from leaf_p2m_kernel), and
+// starts at each internal node whose children are all leaves (pending -1; their moments come from leaf_p2m_kernel), and
 // the block that completes a node's last internal child goes on to the node itself (no level barriers, no
 // waits).  Writers fence before the counter's decrement and the next block reads the children through L2.
 
@@ -247,32 +247,46 @@ __device__ __forceinline__ double4 ldcg4(const double4* p) {
     return make_double4(a.x, a.y, b.x, b.y);
 }
 
-constexpr int kM2mThreads = 256;
+// A block takes one launch position in every gridDim of the node list and finds its starting nodes with one check per
+// thread.  A node costs a chain of short phases (children's data, coefficients, three shifts, result), so they are kept
+// short: the products C(k, j) d^(k-j) are formed once per child and axis, the positions of a shift's terms follow by
+// additions (packed order).  With the products formed and a position table read per term, 256 threads, and tables loaded
+// by every block of the grid before it looked for work, the pass took 70 us on 378 nodes at order 8 (now 50), 113 at order
+// 11 (67), 273 on 7,119 nodes at order 11 (160), 191 on 20,353 nodes of the Poisson kernel at order 7 (142).
+constexpr int kM2mThreads = 512;
+constexpr int kM2mTri = (kPMax + 1) * (kPMax + 2) / 2;  // (k, j <= k) at k (k + 1) / 2 + j
+__host__ __device__ constexpr size_t m2m_smem(int n_mono) {  // child moments and their partial shifts, coefficients
+    return sizeof(double) * ((size_t)16 * n_mono + 8 * 3 * kM2mTri);
+}
 __global__ void __launch_bounds__(kM2mThreads) m2m_upward_kernel(Octree t, int pm, const int4* __restrict__ mono,
                                                          int n_mono, double4* __restrict__ node_ctr,
                                                          double* __restrict__ node_wabs,
                                                          double* __restrict__ node_mom, int heavy_cap,
                                                          int32_t* __restrict__ pending) {
-    extern __shared__ double m2m_sh[];  // 2 x 8 x n_mono: child moments and their partial shifts
+    extern __shared__ double m2m_sh[];
     __shared__ double dp[8][3][kPMax + 1];
-    __shared__ double bin[kPMax + 1][kPMax + 1];
-    __shared__ int mono_idx[kPMax + 1][kPMax + 1][kPMax + 1];  // (a, b, c) -> position in the monomial list
-    __shared__ int climb;
+    __shared__ int climb, n_starts;
+    __shared__ int starts[kM2mThreads];
     __shared__ double4 ch[8];  // the current node's children: centres (w = radius), counts, sum |w|
     __shared__ double chm[8], chw[8];
-    for (int i = threadIdx.x; i < (kPMax + 1) * (kPMax + 1); i += blockDim.x)
-        bin[i / (kPMax + 1)][i % (kPMax + 1)] = c_binom[i / (kPMax + 1)][i % (kPMax + 1)];
-    for (int i = threadIdx.x; i < n_mono; i += blockDim.x) {
-        const int4 k = mono[i];
-        mono_idx[k.x][k.y][k.z] = i;
-    }
-    __syncthreads();
+    __shared__ double bin[kM2mTri];  // C(k, j), filled by a block that has work
+    bool filled = false;
+    double* const S0 = m2m_sh;                 // nc x n_mono
+    double* const S1 = m2m_sh + 8 * n_mono;    // nc x n_mono
+    double* const cf = m2m_sh + 16 * n_mono;   // [child][axis][tri]
+    const int nn = t.counters[1];
     // one internal node (block-wide); the children's centres, weights and moments were written by other
     // blocks of this launch (or by leaf_p2m_kernel) and are read past L1
     auto m2m_node = [&](int node) {
         const int nc = t.node_nchild[node];
         const int fc = t.node_first_child[node];
         __syncthreads();  // the previous node's readers of ch / dp / m2m_sh are done
+        const bool moments = fc + nc <= heavy_cap;  // uniform per block: else a child (numbered after node) has none
+        if (moments) {
+            const double* cm = node_mom + (size_t)fc * n_mono;  // the children are consecutive nodes
+#pragma unroll 4
+            for (int i = threadIdx.x; i < nc * n_mono; i += kM2mThreads) S0[i] = __ldcg(cm + i);
+        }
         if ((int)threadIdx.x < nc) {  // the children's centres, counts and weights, one thread each
             ch[threadIdx.x] = ldcg4(node_ctr + fc + threadIdx.x);
             chm[threadIdx.x] = (double)(t.node_end[fc + threadIdx.x] - t.node_start[fc + threadIdx.x]);
@@ -285,16 +299,16 @@ __global__ void __launch_bounds__(kM2mThreads) m2m_upward_kernel(Octree t, int p
             wabs += chw[k];
         }
         cx /= cnt; cy /= cnt; cz /= cnt;
-        double r = 0;
-        for (int k = 0; k < nc; ++k) {
-            const double dx = ch[k].x - cx, dy = ch[k].y - cy, dz = ch[k].z - cz;
-            r = fmax(r, sqrt(dx * dx + dy * dy + dz * dz) + ch[k].w);
-        }
         if (threadIdx.x == 0) {
+            double r = 0;
+            for (int k = 0; k < nc; ++k) {
+                const double dx = ch[k].x - cx, dy = ch[k].y - cy, dz = ch[k].z - cz;
+                r = fmax(r, sqrt(dx * dx + dy * dy + dz * dz) + ch[k].w);
+            }
             node_ctr[node] = make_double4(cx, cy, cz, r);
             node_wabs[node] = wabs;
         }
-        if (fc + nc > heavy_cap) return;  // uniform per block: a child (numbered after node) has no moments
+        if (!moments) return;
         if (threadIdx.x < nc * 3) {
             const int k = threadIdx.x / 3, a = threadIdx.x % 3;
             const double4 cc = ch[k];
@@ -305,61 +319,98 @@ __global__ void __launch_bounds__(kM2mThreads) m2m_upward_kernel(Octree t, int p
                 v *= d;
             }
         }
-        double* S0 = m2m_sh;                  // nc x n_mono
-        double* S1 = m2m_sh + 8 * n_mono;     // nc x n_mono
-        const double* cm = node_mom + (size_t)fc * n_mono;  // the children are consecutive nodes
-#pragma unroll 4
-        for (int i = threadIdx.x; i < nc * n_mono; i += blockDim.x) S0[i] = __ldcg(cm + i);
+        __syncthreads();
+        const int tri = (pm + 1) * (pm + 2) / 2;
+        for (int i = threadIdx.x; i < nc * 3 * tri; i += kM2mThreads) {
+            const int ca = i / tri, q = i - ca * tri;
+            int k = (int)((sqrtf(8.0f * (float)q + 1.0f) - 1.0f) * 0.5f);  // k (k + 1) / 2 <= q
+            k += (k + 1) * (k + 2) / 2 <= q;
+            k -= k * (k + 1) / 2 > q;
+            const int j = q - k * (k + 1) / 2;
+            cf[ca * kM2mTri + q] = bin[q] * dp[ca / 3][ca % 3][k - j];
+        }
         __syncthreads();
         // the shift factorises by axis: three 1D binomial shifts (x, then y, then z with the sum over
         // children), (k_x + 1) + (k_y + 1) + (k_z + 1) terms per monomial instead of their product
-        for (int i = threadIdx.x; i < nc * n_mono; i += blockDim.x) {
+        for (int i = threadIdx.x; i < nc * n_mono; i += kM2mThreads) {
             const int k = i / n_mono, term = i - k * n_mono;
             const int4 kk = mono[term];
+            const double* c = cf + (k * 3 + 0) * kM2mTri + kk.x * (kk.x + 1) / 2;
+            // (j, k_y, k_z) in packed order: from one j to the next a whole slice, one row step shorter per k_y
+            int at = k * n_mono + kk.y * (pm + 1) - kk.y * (kk.y - 1) / 2 + kk.z;
+            int slice = (pm + 1) * (pm + 2) / 2 - kk.y, row = pm + 1;
             double acc = 0;
-            for (int j0 = 0; j0 <= kk.x; ++j0)
-                acc = fma(bin[kk.x][j0] * dp[k][0][kk.x - j0], S0[k * n_mono + mono_idx[j0][kk.y][kk.z]], acc);
+#pragma unroll 4
+            for (int j = 0; j <= kk.x; ++j) {
+                acc = fma(c[j], S0[at], acc);
+                at += slice;
+                slice -= row;
+                --row;
+            }
             S1[i] = acc;
         }
         __syncthreads();
-        for (int i = threadIdx.x; i < nc * n_mono; i += blockDim.x) {
+        for (int i = threadIdx.x; i < nc * n_mono; i += kM2mThreads) {
             const int k = i / n_mono, term = i - k * n_mono;
             const int4 kk = mono[term];
+            const double* c = cf + (k * 3 + 1) * kM2mTri + kk.y * (kk.y + 1) / 2;
+            int at = k * n_mono + mono_index(kk.x, 0, kk.z, pm), row = pm - kk.x + 1;
             double acc = 0;
-            for (int j1 = 0; j1 <= kk.y; ++j1)
-                acc = fma(bin[kk.y][j1] * dp[k][1][kk.y - j1], S1[k * n_mono + mono_idx[kk.x][j1][kk.z]], acc);
+#pragma unroll 4
+            for (int j = 0; j <= kk.y; ++j) {
+                acc = fma(c[j], S1[at], acc);
+                at += row;
+                --row;
+            }
             S0[i] = acc;
         }
         __syncthreads();
         double* mout = node_mom + (size_t)node * n_mono;
-        for (int term = threadIdx.x; term < n_mono; term += blockDim.x) {
+        for (int term = threadIdx.x; term < n_mono; term += kM2mThreads) {
             const int4 kk = mono[term];
+            const int first = term - kk.z;  // (k_x, k_y, 0)
             double acc = 0;
-            for (int k = 0; k < nc; ++k)
-                for (int j2 = 0; j2 <= kk.z; ++j2)
-                    acc = fma(bin[kk.z][j2] * dp[k][2][kk.z - j2], S0[k * n_mono + mono_idx[kk.x][kk.y][j2]], acc);
+            for (int k = 0; k < nc; ++k) {
+                const double* c = cf + (k * 3 + 2) * kM2mTri + kk.z * (kk.z + 1) / 2;
+                const double* s = S0 + k * n_mono + first;
+#pragma unroll 4
+                for (int j = 0; j <= kk.z; ++j) acc = fma(c[j], s[j], acc);
+            }
             mout[term] = acc;
         }
     };
-    const int nn = t.counters[1];
-    for (int start = blockIdx.x; start < nn; start += gridDim.x) {
-        const int nc = t.node_nchild[start];
-        bool first = nc > 0;  // an internal node whose children are all leaves (uniform per block)
-        for (int k = 0; k < nc; ++k) first = first && t.node_nchild[t.node_first_child[start] + k] == 0;
-        if (!first) continue;
-        for (int node = start;;) {
-            m2m_node(node);
-            __threadfence();  // this thread's writes of node's data before the counter moves
-            __syncthreads();
-            const int parent = t.node_parent[node];
-            if (parent < 0) break;  // uniform: the root
-            if (threadIdx.x == 0) {
-                climb = atomicSub(pending + parent, 1) == 1;  // the parent's last internal child
-                __threadfence();
+    // starting nodes: internal nodes whose children are all leaves
+    for (int64_t base = blockIdx.x; base < nn; base += (int64_t)gridDim.x * kM2mThreads) {
+        __syncthreads();
+        if (threadIdx.x == 0) n_starts = 0;
+        __syncthreads();
+        const int64_t node = base + (int64_t)threadIdx.x * gridDim.x;
+        if (node < nn && __ldcg(pending + node) < 0) starts[atomicAdd(&n_starts, 1)] = (int)node;
+        __syncthreads();
+        const int n = n_starts;
+        if (n > 0 && !filled) {  // uniform per block; m2m_node's barriers order it before its readers
+            filled = true;
+            if (threadIdx.x < kM2mTri) {
+                int k = 0;
+                while ((k + 1) * (k + 2) / 2 <= (int)threadIdx.x) ++k;
+                bin[threadIdx.x] = c_binom[k][threadIdx.x - k * (k + 1) / 2];
             }
-            __syncthreads();
-            if (!climb) break;
-            node = parent;
+        }
+        for (int i = 0; i < n; ++i) {
+            for (int node = starts[i];;) {
+                m2m_node(node);
+                __threadfence();  // this thread's writes of node's data before the counter moves
+                __syncthreads();
+                const int parent = t.node_parent[node];
+                if (parent < 0) break;  // uniform: the root
+                if (threadIdx.x == 0) {
+                    climb = atomicSub(pending + parent, 1) == 1;  // the parent's last internal child
+                    __threadfence();
+                }
+                __syncthreads();
+                if (!climb) break;
+                node = parent;
+            }
         }
     }
 }
@@ -2940,7 +2991,7 @@ int tree_solver_create(lpm_ctx* ctx, const lpm_kernel_desc& kernel, const lpm_so
         const int mono_max = (kPMax + 1) * (kPMax + 2) * (kPMax + 3) / 6;
         if (ea == cudaSuccess)
             ea = cudaFuncSetAttribute(m2m_upward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)(16 * mono_max * sizeof(double)));
+                                      (int)m2m_smem(mono_max));
         if (ea != cudaSuccess) {
             tree_solver_destroy(t);
             return cuda_status(ea, "cudaFuncSetAttribute (far_kernel)");
@@ -3182,7 +3233,7 @@ static int tree_prepare(TreeSolver* t, const double4* src, int64_t n_src, const 
     LPM_LAUNCH(ctx, "leaf_p2m_kernel", leaf_p2m_kernel, gl, kP2mThreads, 0, t->st, t->src_sorted, t->pm, t->p2m_units,
                t->n_units,
                t->node_ctr, t->node_wabs, t->node_mom, t->src32, t->scalar ? 1.0 : 2.0, t->heavy_cap);
-    LPM_LAUNCH(ctx, "m2m_upward_kernel", m2m_upward_kernel, gl, kM2mThreads, (size_t)16 * t->n_mono * sizeof(double), t->st,
+    LPM_LAUNCH(ctx, "m2m_upward_kernel", m2m_upward_kernel, gl, kM2mThreads, m2m_smem(t->n_mono), t->st,
                t->pm, t->mono, t->n_mono, t->node_ctr, t->node_wabs, t->node_mom, t->heavy_cap, t->m2m_pending);
     // far-field coefficients: needed only by the far kernels, so (profiling off) on the side stream during the
     // node features and the traversal
