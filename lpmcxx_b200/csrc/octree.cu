@@ -128,6 +128,47 @@ __device__ __forceinline__ int32_t cluster_excl(int32_t v, int32_t* slot, int ra
     return before;
 }
 
+// In-place exclusive scan of m counts (a multiple of 4, 16-byte aligned) by one cluster: a warp's consecutive runs of
+// 128 are summed, the warp sums scanned over the block and the cluster, and the runs scanned on their second read.
+__global__ void __cluster_dims__(kClBlocks, 1, 1) __launch_bounds__(kClThreads)
+    cluster_scan_kernel(int32_t* __restrict__ data, int m) {
+    __shared__ int32_t slot, warp_base[kClThreads / 32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, rank = (int)blockIdx.x;
+    const int per = (m + 128 * kClWarps - 1) / (128 * kClWarps);  // runs a warp
+    const int b = (rank * (kClThreads / 32) + w) * per;
+    int4* const d4 = (int4*)data;
+    int32_t sum = 0;
+    for (int r = b; r < b + per; ++r) {
+        const int i = 32 * r + lane;
+        const int4 v = 4 * i < m ? d4[i] : make_int4(0, 0, 0, 0);
+        sum += v.x + v.y + v.z + v.w;
+    }
+    sum = warp_incl_scan(sum);
+    if (lane == 31) warp_base[w] = sum;
+    __syncthreads();
+    int32_t block_total = 0, all = 0;
+    const int32_t mine = threadIdx.x < kClThreads / 32 ? warp_base[threadIdx.x] : 0;
+    int32_t base = block_excl_scan(mine, &block_total);
+    base += cluster_excl(block_total, &slot, rank, &all);
+    if (threadIdx.x < kClThreads / 32) warp_base[threadIdx.x] = base;
+    __syncthreads();
+    int32_t run = warp_base[w];
+    for (int r = b; r < b + per; ++r) {
+        const int i = 32 * r + lane;
+        int4 v = 4 * i < m ? d4[i] : make_int4(0, 0, 0, 0);
+        const int32_t s = v.x + v.y + v.z + v.w, incl = warp_incl_scan(s);
+        int32_t at = run + incl - s;
+        const int32_t x = v.x, y = v.y, z = v.z;
+        v.x = at;
+        v.y = at += x;
+        v.z = at += y;
+        v.w = at + z;
+        if (4 * i < m) d4[i] = v;
+        run += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    cluster_barrier();  // no block leaves while another reads its total
+}
+
 // ---------------------------------------------------------------------------------- radix sort
 template <typename K>
 __global__ void __launch_bounds__(kSortThreads) radix_hist_kernel(const K* __restrict__ keys, int64_t n, int shift,
@@ -382,11 +423,16 @@ __global__ void __launch_bounds__(kSortThreads) packed_scatter_kernel(const uint
     }
 }
 
-// Digit counts of every tile to global offsets; a single block suffices for small arrays, the three-pass scan takes
-// the large ones (1.3M keys: 256 x 320 counts).
+// Digit counts of every tile to global offsets.  One launch where the counts allow it: a block for up to 4096 (4.4 us
+// against 6.3 us by a cluster; 10.4 and 20.8 us at 8,192 and 16,384), a cluster up to 2^19 (6.4 us at 65,536 counts, the
+// 1M keys of a pass, against 12.4 us back to back by the three launches; equal at 2^19, 20.9 against 16.5 us at 2^20).
+constexpr int64_t kBlockScanMax = 4096, kClusterScanMax = 1 << 19;
 int digit_offsets(lpm_ctx* ctx, int32_t* counts, int64_t m, int sums_slot) {
-    if (m > 16 * 1024) return scan_exclusive_i32(ctx, counts, counts, m, nullptr, sums_slot);
-    LPM_LAUNCH(ctx, "scan_single_block_kernel", scan_single_block_kernel, 1, 1024, 0, counts, m, (int32_t*)nullptr);
+    if (m > kClusterScanMax) return scan_exclusive_i32(ctx, counts, counts, m, nullptr, sums_slot);
+    if (m > kBlockScanMax)
+        LPM_LAUNCH(ctx, "cluster_scan_kernel", cluster_scan_kernel, kClBlocks, kClThreads, 0, counts, (int)m);
+    else
+        LPM_LAUNCH(ctx, "scan_single_block_kernel", scan_single_block_kernel, 1, 1024, 0, counts, m, (int32_t*)nullptr);
     return LPM_OK;
 }
 
@@ -431,9 +477,14 @@ int radix_sort_impl(lpm_ctx* ctx, K* keys, int32_t* vals, K* tk, int32_t* tv, in
 }
 
 // ---------------------------------------------------------------------------------- keys
+// Packed keys keep 32 bits of the key, which are 11 of the 21 levels' digits.  The count of points inside goes out once
+// a block: one addition a warp, all on the same address, took half the time of 1M points (38 -> 24 us with both).
+constexpr int kPackedLevels = (31 + 2) / 3;
+static_assert(3 * (kKeyLevels - kPackedLevels) <= 32, "the levels left out lie in the lower half of the key");
 __global__ void morton_keys_kernel(const double4* __restrict__ pts, int64_t n, RootBox root,
                                    uint64_t* __restrict__ keys, int32_t* __restrict__ vals,
                                    int32_t* __restrict__ counters, int bits, int max_depth, bool packed) {
+    const int levels = packed ? kPackedLevels : kKeyLevels;  // (bits == 1 stops at max_depth)
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     root = resolve_root(root);
     bool in = false;
@@ -461,7 +512,7 @@ __global__ void morton_keys_kernel(const double4* __restrict__ pts, int64_t n, R
             double lo[3] = {root.lo[0], root.lo[1], root.lo[2]};
             double hi[3] = {root.hi[0], root.hi[1], root.hi[2]};
             key = 0;
-            for (int l = 1; l <= kKeyLevels; ++l) {
+            for (int l = 1; l <= levels; ++l) {
                 uint64_t digit = 0;
 #pragma unroll
                 for (int a = 0; a < 3; ++a) {
@@ -483,8 +534,8 @@ __global__ void morton_keys_kernel(const double4* __restrict__ pts, int64_t n, R
             vals[i] = (int32_t)i;
         }
     }
-    const unsigned b = __ballot_sync(0xffffffffu, in);
-    if ((threadIdx.x & 31) == 0 && b) atomicAdd(&counters[0], __popc(b));
+    const int inside = __syncthreads_count(in);
+    if (threadIdx.x == 0 && inside) atomicAdd(&counters[0], inside);
 }
 
 __global__ void root_extent_kernel(const double4* __restrict__ pts, int64_t first, int64_t n, int mode,

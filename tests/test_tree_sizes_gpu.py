@@ -54,3 +54,14 @@ def test_poisson_treecode_at_batch_cut_boundaries(ctx, n):
         assert torch.isfinite(out).all()
         assert float((out - ref).norm()) <= 5e-6 * float(ref.norm())
     ts.close()
+
+
+@pytest.mark.parametrize("n,depth", [(65536, 21), (65537, 21), (524288, 10), (524289, 10), (700001, 21)])
+def test_tree_at_digit_scan_boundaries(ctx, n, depth):
+    """The digit counts of a many-block pass, 256 per 4096 keys, scanned by a block (65,536 pairs), by a cluster with one
+    run of 128 a warp (up to 524,288 keys) and with several."""
+    torch = ctx.use_torch_stream()
+    pts = _points(n, n)
+    tree = L.Tree(ctx, torch.tensor(pts, device="cuda"), BOX, 200, depth, allow_overflow=True)
+    _check(tree, oracle.tree_build(pts, BOX, 200, depth))
+    tree.close()
