@@ -171,13 +171,13 @@ __global__ void __launch_bounds__(128) mlp_predict_bf16_kernel(const __nv_bfloat
                                                                const float* __restrict__ norm,
                                                                const float* __restrict__ feats, int64_t n,
                                                                int32_t* __restrict__ cls) {
-    __shared__ __align__(16) __nv_bfloat16 xs[4][32 * 16];
+    __shared__ __align__(16) __nv_bfloat16 xs[4][32 * kMlpIn];
     const int64_t base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31);
     if (base >= n) return;  // uniform per warp
     const int64_t i = base + (threadIdx.x & 31);
     float f[kMlpIn];
     for (int k = 0; k < kMlpIn; ++k) f[k] = i < n ? feats[i * kMlpIn + k] : norm[k];
-    const int c = mlp_warp_argmax(w, norm, f, xs[threadIdx.x >> 5]);
+    const int c = mlp_warp_argmax<0>(w, norm, f, xs[threadIdx.x >> 5], threadIdx.x & 31, (int)min((int64_t)32, n - base));
     if (i < n) cls[i] = c;
 }
 

@@ -545,7 +545,6 @@ struct TraverseArgs {
     double theta;
     int order;
     int direct_below;
-    int fill;  // 0 = count, 1 = fill
     int32_t* far_cnt;  // far lists are bucketed by order: row P (stride nb1) holds every batch's order-P entries
     int32_t* near_cnt;
     const int32_t* far_off;
@@ -575,6 +574,9 @@ struct TraverseArgs {
 
 constexpr int kWarpStack = 1024;
 constexpr int kDecisionCap = 1024;  // cached selector decisions per batch
+constexpr int kMlpPad = 8;             // MlpLayout of the selector's weights in shared memory
+constexpr int kOrderBits = 4;         // an order fits
+static_assert(kPMax < 1 << kOrderBits, "orders are told apart by kOrderBits ballots");
 
 // ---------------------------------------------------------------------------------- learned order
 // Per node: log10 radius, log10 sum|w|, log10 of the Frobenius norms of the degree-2/4/6 moment tensors
@@ -631,36 +633,52 @@ __device__ __forceinline__ float log_budget(const double* node_wabs, double eps)
     return (float)log10(2.0 / fmax(eps * node_wabs[0], 1e-300));
 }
 
+// The selector in the fill pass, which meets more than kDecisionCap accepted clusters in a batch rarely: on the weights
+// in global memory, and out of line for the registers of the pass.
+__device__ __noinline__ int selector_class_again(const __nv_bfloat16* __restrict__ w, const float* norm, const float* f,
+                                                 __nv_bfloat16* xs, int row, int rows) {
+    return mlp_warp_argmax<0>(w, norm, f, xs, row, rows);
+}
+
 // One warp per target batch walks the source tree breadth-first, up to 32 nodes per step: (batch, node)
 // pairs that pass the acceptance test go to the far list with the order to use; leaves that fail it,
 // and accepted clusters too small to be worth an expansion, go to the near list as leaf-id ranges.
 // Entries are appended in lane order, so the lists are deterministic.
-// Registers capped for 4 resident blocks per SM (16 warps): the count pass, which runs the selector MLP,
-// is latency-bound, and at its natural 140 registers only 3 blocks fit (measured 1.52 -> 1.43 ms at icos L8).
-#ifndef LPM_TRAVERSE_MIN_BLOCKS
-#define LPM_TRAVERSE_MIN_BLOCKS 4
-#endif
-__global__ void __launch_bounds__(128, LPM_TRAVERSE_MIN_BLOCKS) traverse_kernel(TraverseArgs A) {
+// Bound by the latency of its steps (a round of loads, the test, the appends), so what a pass does not do is compiled
+// out of it: without the selector 44 (fill) and 59 (count) registers instead of 128 and no weights in shared memory
+// let twice the warps hide each other's steps (both passes 243 -> 123 us for 1M Poisson targets, 32 -> 25 us for 50k).
+// The selector's count pass is bound by the activations: 122 registers at 4 blocks per SM (5 and 6 blocks spill: 578 ->
+// 607, 630 us at 1.3M targets and order selection; with unpadded weight rows, staged one value at a time, and 32 rows
+// evaluated for every step it took 800 us).
+template <bool kLearned, bool kFill>
+__global__ void __launch_bounds__(128, kLearned && !kFill ? 4 : 8) traverse_kernel(TraverseArgs A) {
     __shared__ int sstack[4][kWarpStack];
-    __shared__ int pcnt[4][kPMax + 1];  // per warp: far entries of each order so far
-    __shared__ __align__(16) __nv_bfloat16 mw[kMlpParams];
-    __shared__ __align__(16) __nv_bfloat16 mxs[4][32 * 16];  // per warp: the selector's input rows
+    __shared__ int pcnt[4][kPMax + 1];  // per warp: far entries of each order so far (fill: the next one's place)
+    // the selector's weights; the fill pass runs it past kDecisionCap only, on the weights in global memory
+    __shared__ __align__(16) __nv_bfloat16 mw[kLearned && !kFill ? MlpLayout<kMlpPad>::kSize : 8];
+    __shared__ __align__(16) __nv_bfloat16 mxs[4][kLearned ? 32 * kMlpIn : 8];  // per warp: the selector's input rows
     __shared__ float mnorm[2 * kMlpIn];
-    if (A.learned) {  // uniform per launch
-        for (int i = threadIdx.x; i < kMlpParams; i += blockDim.x) mw[i] = A.mlp_w[i];
+    __shared__ unsigned long long block_pairs[3];  // pair_counts of the warps done so far
+    __shared__ int warps_done;
+    if (threadIdx.x < 3) block_pairs[threadIdx.x] = 0;
+    if (threadIdx.x == 3) warps_done = 0;
+    if constexpr (kLearned) {
+        if (!kFill) mlp_stage<kMlpPad>(A.mlp_w, mw);
         for (int i = threadIdx.x; i < 2 * kMlpIn; i += blockDim.x) mnorm[i] = A.mlp_norm[i];
-        __syncthreads();
     }
+    __syncthreads();
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t b = (int64_t)blockIdx.x * 4 + w;
-    if (A.fill && b == 0 && lane == 0 && A.t.counters[1] > A.heavy_cap) atomicOr(&A.flags[0], 16);
+    if (kFill && b == 0 && lane == 0 && A.t.counters[1] > A.heavy_cap) atomicOr(&A.flags[0], 16);
     if (b >= A.n_batches) return;  // uniform per warp
+    // batches of this block, the warps that add to its pair counts
+    const int live = (int)max((int64_t)0, min((int64_t)4, min((int64_t)*A.nbat, A.n_batches) - 4 * (int64_t)blockIdx.x));
     const Octree& t = A.t;
     const unsigned full = 0xffffffffu, lt = (1u << lane) - 1u;
     int* st = sstack[w];
-    if (lane <= kPMax) pcnt[w][lane] = 0;
+    if (lane <= kPMax) pcnt[w][lane] = kFill && b < *A.nbat ? A.far_off[lane * A.nb1 + b] : 0;
     if (t.counters[1] == 0 || t.counters[0] == 0 || b >= *A.nbat) {
-        if (!A.fill) {
+        if (!kFill) {
             if (lane <= kPMax) A.far_cnt[lane * A.nb1 + b] = 0;
             if (lane == 0) {
                 A.near_cnt[b] = 0;
@@ -672,13 +690,14 @@ __global__ void __launch_bounds__(128, LPM_TRAVERSE_MIN_BLOCKS) traverse_kernel(
     }
     const double4 bc = A.batch_ctr[b];
     const unsigned long long nb = (unsigned long long)(A.batch_first[b + 1] - A.batch_first[b]);
-    const float log_s = A.learned ? log_budget(A.node_wabs, A.eps) : 0.0f;
+    const float log_s = kLearned ? log_budget(A.node_wabs, A.eps) : 0.0f;
     int size = 1;
     if (lane == 0) st[0] = 0;
     __syncwarp();
     int nnear = 0, ndec = 0;
     unsigned long long far_pairs = 0, near_pairs = 0, far_terms = 0;
-    const int64_t noff = A.fill ? A.near_off[b] : 0;
+    const int64_t noff = kFill ? A.near_off[b] : 0;
+    // far_pairs is the warp's, near_pairs and far_terms are this lane's until the walk is over
     while (size > 0) {
         const int m = min(32, size);
         const int node = lane < m ? st[size - 1 - lane] : -1;
@@ -686,19 +705,22 @@ __global__ void __launch_bounds__(128, LPM_TRAVERSE_MIN_BLOCKS) traverse_kernel(
         size -= m;
         int kind = 0, nch = 0, lo = 0, hi = 0, cnt = 0, fc = 0, P = A.order;
         double4 c = make_double4(0, 0, 0, 0);
-        int s = 0, e = 0, nc = 0;
+        int s = 0, e = 0, nc = 0, leaf0 = 0, leaves = 0;
         bool far_ok = false;
         if (node >= 0) {
             c = A.node_ctr[node];
             s = t.node_start[node];
             e = t.node_end[node];
+            nc = t.node_nchild[node];
+            fc = t.node_first_child[node];  // with the leaf range, needed or not: their loads overlap the test
+            leaf0 = t.node_leaf0[node];
+            leaves = t.node_leaves[node];
             const double dx = bc.x - c.x, dy = bc.y - c.y, dz = bc.z - c.z;
             const double R = sqrt(dx * dx + dy * dy + dz * dz);
             far_ok = R > bc.w && c.w < A.theta * (R - bc.w) && node < A.heavy_cap;
-            nc = t.node_nchild[node];
         }
         int cut = A.direct_below;
-        if (A.learned) {  // uniform per launch
+        if constexpr (kLearned) {
             // the selector's order; "no order meets the budget" opens a cluster large enough to be worth
             // opening and sums a leaf or a small cluster directly.  The count pass caches each batch's
             // first kDecisionCap decisions (in visiting order) for the fill pass.
@@ -707,17 +729,18 @@ __global__ void __launch_bounds__(128, LPM_TRAVERSE_MIN_BLOCKS) traverse_kernel(
             ndec += __popc(okm);
             uint8_t* dec = A.decisions + (size_t)b * kDecisionCap;
             int cls = -1;
-            if (far_ok && A.fill && idx < kDecisionCap) cls = dec[idx];
+            if (far_ok && kFill && idx < kDecisionCap) cls = dec[idx];
             const bool need = far_ok && cls < 0;
-            if (__any_sync(full, need)) {  // the whole warp runs the selector on the tensor cores
-                float f[kMlpIn];
-#pragma unroll
-                for (int i = 0; i < kMlpIn; ++i) f[i] = mnorm[i];  // finite filler for lanes without a pair
+            const unsigned needm = __ballot_sync(full, need);
+            if (needm) {  // the whole warp runs the selector on the tensor cores
+                float f[kMlpIn] = {};
                 if (need) pair_features(bc, c, A.node_feat + (size_t)node * kMlpIn, log_s, f);
-                const int c2 = mlp_warp_argmax(mw, mnorm, f, mxs[w]);
+                const int row = need ? __popc(needm & lt) : -1;
+                const int c2 = kFill ? selector_class_again(A.mlp_w, mnorm, f, mxs[w], row, __popc(needm))
+                                     : mlp_warp_argmax<kMlpPad>(mw, mnorm, f, mxs[w], row, __popc(needm));
                 if (need) {
                     cls = c2;
-                    if (!A.fill && idx < kDecisionCap) dec[idx] = (uint8_t)cls;
+                    if (!kFill && idx < kDecisionCap) dec[idx] = (uint8_t)cls;
                 }
             }
             if (far_ok) {
@@ -731,25 +754,31 @@ __global__ void __launch_bounds__(128, LPM_TRAVERSE_MIN_BLOCKS) traverse_kernel(
                 kind = 1;
             } else if (far_ok || nc == 0) {
                 kind = 2;
-                lo = t.node_leaf0[node];
-                hi = lo + t.node_leaves[node] - 1;
+                lo = leaf0;
+                hi = lo + leaves - 1;
                 cnt = e - s;
             } else {
                 kind = 3;
                 nch = nc;
-                fc = t.node_first_child[node];
             }
         }
         const unsigned fm = __ballot_sync(full, kind == 1);
         if (fm) {  // warp-uniform: rank each far entry among this step's entries of its order, in lane order
-            const unsigned grp = __match_any_sync(full, kind == 1 ? P : 64 + lane);
+            unsigned grp = fm;
+            if (kLearned) {
+#pragma unroll
+                for (int bit = 0; bit < kOrderBits; ++bit) {
+                    const unsigned m1 = __ballot_sync(full, (P >> bit) & 1);
+                    grp &= (P >> bit) & 1 ? m1 : ~m1;
+                }
+            }
             const int rank = __popc(grp & lt);
             const int base = kind == 1 ? pcnt[w][P] : 0;
             __syncwarp();
             if (kind == 1) {
                 if (rank == 0) pcnt[w][P] = base + __popc(grp);
-                if (A.fill) {
-                    const int64_t at = A.far_off[P * A.nb1 + b] + base + rank;
+                if (kFill) {
+                    const int64_t at = base + rank;
                     if (at < A.far_cap) A.far_list[at] = make_int2(node, P);
                     else atomicOr(&A.flags[0], 1);
                 }
@@ -758,44 +787,50 @@ __global__ void __launch_bounds__(128, LPM_TRAVERSE_MIN_BLOCKS) traverse_kernel(
         }
         far_pairs += (unsigned long long)__popc(fm) * nb;
         const unsigned nm = __ballot_sync(full, kind == 2);
-        if (kind == 2 && A.fill) {
+        if (kind == 2 && kFill) {
             const int64_t at = noff + nnear + __popc(nm & lt);
             if (at < A.near_cap) A.near_list[at] = make_int2(lo, hi);
             else atomicOr(&A.flags[0], 2);
         }
         nnear += __popc(nm);
-        unsigned long long np = (unsigned long long)cnt * nb;
-        unsigned long long ft = kind == 1 ? (unsigned long long)entries_for(P) * nb : 0ull;
-        for (int o = 16; o > 0; o >>= 1) {
-            np += __shfl_xor_sync(full, np, o);
-            ft += __shfl_xor_sync(full, ft, o);
+        near_pairs += (unsigned long long)cnt * nb;
+        if (kind == 1) far_terms += (unsigned long long)entries_for(P) * nb;
+        // push the children of split nodes: their counts (up to 8) summed over the lanes below bit by bit
+        int before = 0, total = 0;
+#pragma unroll
+        for (int bit = 0; bit < 4; ++bit) {
+            const unsigned m1 = __ballot_sync(full, (nch >> bit) & 1);
+            before += __popc(m1 & lt) << bit;
+            total += __popc(m1) << bit;
         }
-        near_pairs += np;
-        far_terms += ft;
-        // push the children of split nodes
-        int incl = nch;
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(full, incl, o);
-            if (lane >= o) incl += v;
-        }
-        const int total = __shfl_sync(full, incl, 31);
         if (size + total > kWarpStack) {
             if (lane == 0) atomicOr(&A.flags[0], 4);
         } else if (kind == 3) {
-            const int base = size + incl - nch;
+            const int base = size + before;
             for (int k = 0; k < nch; ++k) st[base + k] = fc + nch - 1 - k;
         }
         __syncwarp();
         if (size + total <= kWarpStack) size += total;
     }
-    if (!A.fill && lane <= kPMax) A.far_cnt[lane * A.nb1 + b] = pcnt[w][lane];
-    if (!A.fill && lane == 0) {
+    if (kFill) return;
+    for (int o = 16; o > 0; o >>= 1) {
+        near_pairs += __shfl_xor_sync(full, near_pairs, o);
+        far_terms += __shfl_xor_sync(full, far_terms, o);
+    }
+    if (lane <= kPMax) A.far_cnt[lane * A.nb1 + b] = pcnt[w][lane];
+    if (lane == 0) {
         A.near_cnt[b] = nnear;
         A.near_work[b] = (uint32_t)min(near_pairs, 0xffffffffull);
         A.far_work[b] = (uint32_t)min(far_terms, 0xffffffffull);
-        atomicAdd(&A.pair_counts[0], far_pairs);
-        atomicAdd(&A.pair_counts[1], near_pairs);
-        atomicAdd(&A.pair_counts[2], far_terms);
+        // one global addition a block, by its last warp: three a batch on the same addresses queue up at L2
+        atomicAdd(&block_pairs[0], far_pairs);
+        atomicAdd(&block_pairs[1], near_pairs);
+        atomicAdd(&block_pairs[2], far_terms);
+        __threadfence_block();
+        if (atomicAdd(&warps_done, 1) == live - 1) {
+            __threadfence_block();
+            for (int k = 0; k < 3; ++k) atomicAdd(&A.pair_counts[k], atomicAdd(&block_pairs[k], 0ull));
+        }
     }
 }
 
@@ -3087,7 +3122,6 @@ static int build_lists(TreeSolver* t, bool wait, bool sched) {
     A.near_off = t->near_off;
     A.flags = t->flags;
     A.pair_counts = t->pair_counts;
-    A.fill = 0;
     A.learned = (t->learned && t->mlp_loaded) ? 1 : 0;
     A.max_order = std::min(t->pm, kMlpDirectClass);
     A.order_bias = t->order_bias;
@@ -3102,7 +3136,9 @@ static int build_lists(TreeSolver* t, bool wait, bool sched) {
     A.near_work = t->near_work;
     A.far_work = t->far_work;
     const unsigned g = grid_for(t->n_batches, 4);
-    LPM_LAUNCH(ctx, "traverse_kernel", traverse_kernel, g, 128, 0, A);
+    const auto count = A.learned ? traverse_kernel<true, false> : traverse_kernel<false, false>;
+    const auto fill = A.learned ? traverse_kernel<true, true> : traverse_kernel<false, true>;
+    LPM_LAUNCH(ctx, "traverse_kernel", count, g, 128, 0, A);
     ListsArgs L{};
     L.nbat = t->tcount + 1;
     L.nb1 = t->n_batches + 1;
@@ -3131,12 +3167,11 @@ static int build_lists(TreeSolver* t, bool wait, bool sched) {
             if (rc) return rc;
         }
     }
-    A.fill = 1;
     A.far_list = t->far_list;
     A.near_list = t->near_list;
     A.far_cap = t->far_cap;
     A.near_cap = t->near_cap;
-    LPM_LAUNCH(ctx, "traverse_kernel", traverse_kernel, g, 128, 0, A);
+    LPM_LAUNCH(ctx, "traverse_kernel", fill, g, 128, 0, A);
     return LPM_OK;
 }
 
