@@ -85,8 +85,8 @@ constexpr int kTile = 256;       // sources staged per tile
 // make.  At the end every thread leaves its FP64 sums in shared memory and the cluster's blocks add the G C sums of a
 // target in a fixed order (their own block's and, through distributed shared memory, the others'): the result does
 // not depend on timing, and no workspace is needed.  One block per 512 (FP64) or 1,024 (FP32) targets, as before,
-// left most SMs idle below 10^5 targets: 1,280 sources x 1,922 targets 121 -> 12.4 us, 5,120 x 7,682 482 -> 57.5 us
-// (FP64); 24,576 x 49,154 873 -> 483 us (FP32).
+// left most SMs idle below 10^5 targets: 1,280 sources x 1,922 targets 121 -> 12.3 us, 5,120 x 7,682 482 -> 57.5 us
+// (FP64); 24,576 x 49,154 878 -> 524 us (FP32).
 struct Split {
     int gshift;  // log2 of the thread groups per block
     int parts;   // blocks per cluster = source parts
@@ -250,7 +250,7 @@ struct BsF64 {
 // FP64 Poisson 1/(4 pi r): 12 FP64 operations a pair against 17.  1/r by Householder's third-order step
 // y (1 + e (1/2 + 3/8 e)), e = 1 - r^2 y^2, in place of two Newton steps; a coincident pair (or one whose r^2 is
 // subnormal) adds nothing, by a select of the approximation's high word on the integer pipe (its low word is 0).
-// 20,011 points: 2.85 ms -> 0.37 ms (with the split), 100,011 points 8.5 ms.
+// 20,011 points: 2.85 ms -> 0.35 ms (with the split), 100,011 points 8.5 ms.
 template <int kTPT>
 struct PoissonF64 {
     static constexpr int NC = 1, TPT = kTPT;
@@ -637,10 +637,9 @@ struct PoissonF32 {
     }
 };
 
-// FP32 direct sum, TPT targets per thread (2, 4 or 8; the context's "direct_targets").  A tile of kTile sources is
+// FP32 direct sum, TPT targets per thread (2, 4 or 8: at most the context's "direct_targets").  A tile of kTile sources is
 // always summed by one thread per target in FP32 and folded into FP64 once, so the FP32 sums are the same however
 // the tiles are shared out: every stage holds one tile per group.
-constexpr int kGroups32 = 4;  // most groups per block
 template <class Op, int TPT>
 __global__ void __launch_bounds__(kThreads) direct32_kernel(const float4* __restrict__ src, int64_t n_src,
                                                             const float4* __restrict__ tgt,

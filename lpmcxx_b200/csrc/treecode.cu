@@ -1556,7 +1556,7 @@ __device__ __forceinline__ void far2_batch(const FarArgs& A, int64_t b, float4* 
 }
 
 // far_order_kernel<P, float, float4> with two targets per thread (targets i and i + 64 of the batch):
-// 64 threads per block, stages of kFar2StageUnits, the same double buffering.  Built for 7 blocks per SM
+// 64 threads per block, stages of kFar2StageUnits, list entries a chunk at a time.  Built for 7 blocks per SM
 // (128 registers; the odd orders spill up to 128 bytes to L1) with 768-unit stages: measured faster than
 // 6 blocks without spills, than more resident blocks with smaller stages (fewer block barriers per
 // coefficient) and than fewer blocks with larger ones.
