@@ -2747,7 +2747,10 @@ cudaError_t talloc(TreeSolver* t, Tp** p, size_t count) {
     return e;
 }
 
+// A regrow that fails leaves the solver without the buffers: their capacities are 0 then, so that every kernel's bounds
+// check holds and a later evaluation (or captured replay) flags an overflow instead of writing through a null pointer.
 int alloc_lists(TreeSolver* t, int64_t far_cap, int64_t near_cap) {
+    t->far_cap = t->near_cap = 0;
     for (void** p : {(void**)&t->far_list, (void**)&t->near_list}) {
         if (*p) {
             cudaFree(*p);
@@ -2767,6 +2770,7 @@ int alloc_lists(TreeSolver* t, int64_t far_cap, int64_t near_cap) {
 // Regrow the per-node moment / coefficient / feature arrays to hold `need` nodes (with headroom).
 int heavy_alloc(TreeSolver* t, int64_t need) {
     const int64_t cap = std::min<int64_t>(t->st.node_cap, need + need / 2 + 256);
+    t->heavy_cap = 0;  // until all of them are there (see alloc_lists)
     auto regrow = [&](auto** p, size_t per_node) -> cudaError_t {
         if (*p) {
             cudaFree(*p);
@@ -3504,6 +3508,7 @@ int tree_velocity(TreeSolver* t, const double4* src, int64_t n_src, const double
     // waits: the buffers grow and every output is written again.  (50,021-point Poisson: 501 -> 439 us.)
     for (bool careful = !t->sized;; careful = true) {
         int rc = tree_enqueue(t, src, n_src, X, n_tgt, U, careful);
+        if (rc) t->sized = false;  // a regrow may have failed
         if (rc || n_src == 0 || n_tgt == 0) return rc;
         rc = read_state(t);
         if (rc) return rc;
@@ -3822,6 +3827,9 @@ int tree_get_param(const TreeSolver* t, const char* name, double* value) {
     else if (n == "root_maxr") *value = t->root_maxr;
     else if (n == "root_first") *value = (double)t->root_first;
     else if (n == "order") *value = t->order;
+    else if (n == "far_cap") *value = (double)t->far_cap;
+    else if (n == "near_cap") *value = (double)t->near_cap;
+    else if (n == "heavy_cap") *value = t->heavy_cap;
     else {
         set_error("tree_get_param: unknown parameter %s", name);
         return LPM_ERR_ARG;

@@ -94,3 +94,55 @@ def test_capacity_overflow_in_captured_replay_is_reported_and_recovers(ctx):
     got = rk.get_state()
     rk.close()
     assert np.array_equal(got, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("scalar", [False, True])
+def test_failed_regrow_leaves_the_solver_usable(ctx, scalar):
+    """One solver, sized by an evaluation of particles that sit in one octree cell: each allocation of the regrow that
+    the spread-out particles then need fails in turn.  The call returns LPM_ERR_OOM, at least one of the buffers that
+    went is counted as empty (so that no kernel writes where nothing is), and both inputs evaluate afterwards as on a
+    fresh solver."""
+    torch = ctx.use_torch_stream()
+    _, p, n_src = W.gaussian_vortex_mesh("icos", 5)
+    tiny = p.copy()
+    x0 = np.array([0.0, 0.0, 1.0])
+    tiny[:, :3] = x0 + 1e-9 * (p[:, :3] - x0)
+    tiny[:, :3] /= np.linalg.norm(tiny[:, :3], axis=1, keepdims=True)
+    kernel = L.poisson_kernel() if scalar else L.biot_savart_kernel()
+    solver = L.tree_solver(L.LPM_PREC_F32, 4, 4, 0.3)
+    inputs = [torch.tensor(a, device="cuda") for a in (tiny, p)]
+    comps = 1 if scalar else 3
+
+    def evaluate(ts, d):
+        out = torch.full((comps, p.shape[0]), float("nan"), dtype=torch.float64, device="cuda")
+        ts.eval(d[:n_src], d, out)
+        return out
+
+    want = []
+    for d in inputs:
+        fresh = L.TreeSum(ctx, kernel, solver, n_src, p.shape[0])
+        want.append(evaluate(fresh, d))
+        fresh.close()
+    lib, failed = L.lib(), 0
+    for k in range(20):
+        ts = L.TreeSum(ctx, kernel, solver, n_src, p.shape[0])
+        evaluate(ts, inputs[0])
+        try:
+            lib.lpm_debug_fail_allocations(k)
+            evaluate(ts, inputs[1])
+            done = True
+        except L.LpmError as e:
+            assert e.code == L._capi.LPM_ERR_OOM, (k, e)
+            done = False
+        finally:
+            lib.lpm_debug_fail_allocations(-1)
+        if not done:
+            assert 0 in [ts.get_param(c) for c in ("far_cap", "near_cap", "heavy_cap")]
+            failed += 1
+        for i in (0, 1, 0):
+            assert torch.equal(evaluate(ts, inputs[i]), want[i]), (k, i)
+        ts.close()
+        if done:
+            break
+    assert done and failed >= 2
