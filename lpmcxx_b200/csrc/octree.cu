@@ -830,7 +830,8 @@ __global__ void __cluster_dims__(kClBlocks, 1, 1) __launch_bounds__(kClThreads)
     });
     if (tid == 0) {
         if (total <= cap) batch_first[total] = n;
-        *nbat = total;
+        nbat[0] = (int32_t)min((int64_t)total, cap);
+        nbat[1] = total;
     }
     cluster_barrier();  // no block leaves while another reads its total
 }

@@ -14,8 +14,9 @@ constexpr uint64_t kKeyOutside = ~0ull;
 int scan_exclusive_i32(lpm_ctx* ctx, const int32_t* in, int32_t* out, int64_t n, int32_t* total_dev,
                        int sums_slot = kSlotMisc2);
 
-// Cuts n sorted keys into batches of at most `batch` keys of one cell (keys >> shift): batch_first[0 .. *nbat - 1] their
-// starts, batch_first[*nbat] = n (entries up to index cap), by one launch; false (nothing done) for large n.
+// Cuts n sorted keys into batches of at most `batch` keys of one cell (keys >> shift): batch_first[0 .. nbat[0] - 1]
+// their starts, batch_first[nbat[0]] the last one's end, by one launch; false (nothing done) for large n.  nbat[0] is at
+// most cap, so that its readers stay within arrays of cap batches; nbat[1] is the number there would be.
 bool batch_cut(lpm_ctx* ctx, const uint64_t* keys, int64_t n, int shift, int batch, int32_t* batch_first, int32_t* nbat,
                int64_t cap, int* rc);
 // Stable LSD radix sort of (key, value) pairs over key bits [0, bits), 8 bits per pass, in place (ping-pong through

@@ -499,15 +499,18 @@ __global__ void batch_flags_kernel(const uint64_t* __restrict__ keys, int64_t n,
     }
 }
 
-// batch_first[b] = first sorted target of batch b (b < n_batches), batch_first[n_batches] = n; the number
-// of batches goes to *nbat.  bscan is the exclusive scan of bflag over n + 1 entries.
+// batch_first[b] = first sorted target of batch b (b < nbat[0]), batch_first[nbat[0]] = its end; nbat as batch_cut
+// leaves it.  bscan is the exclusive scan of bflag over n + 1 entries.
 __global__ void batch_first_kernel(const int32_t* __restrict__ bscan, int64_t n, int32_t* __restrict__ batch_first,
                                    int32_t* __restrict__ nbat, int64_t cap) {
     for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q <= n; q += (int64_t)gridDim.x * blockDim.x) {
         const int32_t b = bscan[q];
         const bool start = q == n || bscan[q + 1] != b;
         if (start && b <= cap) batch_first[b] = (int32_t)q;
-        if (q == n) *nbat = b;
+        if (q == n) {
+            nbat[0] = (int32_t)min((int64_t)b, cap);
+            nbat[1] = b;
+        }
     }
 }
 
@@ -2662,7 +2665,7 @@ struct TreeSolver {
     int32_t* tperm = nullptr;
     uint64_t* ttmpk = nullptr;
     int32_t* ttmpv = nullptr;
-    int32_t* tcount = nullptr;
+    int32_t* tcount = nullptr;  // targets inside the root box, batches, batches without the capacity's bound
     double4* tgt_sorted = nullptr;
     double4* batch_ctr = nullptr;
     // sources and nodes
@@ -3746,8 +3749,8 @@ static int state_status(const TreeSolver* t) {
                   "4 traversal stack, 16 node moments); run one uncaptured evaluation to regrow", f[0]);
         return LPM_ERR_CAPACITY;
     }
-    if (tc[1] > t->n_batches) {
-        set_error("tree solver: %d target batches exceed the capacity of %lld", tc[1], (long long)t->n_batches);
+    if (tc[2] > t->n_batches) {
+        set_error("tree solver: %d target batches exceed the capacity of %lld", tc[2], (long long)t->n_batches);
         return LPM_ERR_CAPACITY;
     }
     if (c[2] & 2) {
@@ -3827,6 +3830,7 @@ int tree_get_param(const TreeSolver* t, const char* name, double* value) {
     else if (n == "root_maxr") *value = t->root_maxr;
     else if (n == "root_first") *value = (double)t->root_first;
     else if (n == "order") *value = t->order;
+    else if (n == "batch_cap") *value = (double)t->n_batches;
     else if (n == "far_cap") *value = (double)t->far_cap;
     else if (n == "near_cap") *value = (double)t->near_cap;
     else if (n == "heavy_cap") *value = t->heavy_cap;

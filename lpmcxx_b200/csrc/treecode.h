@@ -53,8 +53,8 @@ int tree_stats(TreeSolver* t, int64_t* out10);
 // (octree level whose cells target batches may not straddle; 1 .. the level chosen at creation), "order_bias"
 // (learned solvers only), "root_maxr" / "root_first" (the root box of the source octree, see TreeSolver).
 int tree_set_param(TreeSolver* t, const char* name, double value);
-// Current value of a run-time parameter (as tree_set_param, plus "batch_level_max", "order" and the entries that the
-// interaction lists ("far_cap", "near_cap") and the nodes that the moment arrays ("heavy_cap") hold).
+// Current value of a run-time parameter (as tree_set_param, plus "batch_level_max", "order" and what the buffers
+// hold: batches "batch_cap", interaction list entries "far_cap" and "near_cap", nodes with moments "heavy_cap").
 int tree_get_param(const TreeSolver* t, const char* name, double* value);
 // Learned order: load the selector (LPM_MLP_PARAMS floats, host) or null for the fixed-order fallback.
 int tree_set_mlp(TreeSolver* t, const float* params_host);

@@ -146,3 +146,29 @@ def test_failed_regrow_leaves_the_solver_usable(ctx, scalar):
         if done:
             break
     assert done and failed >= 2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [110000, 200000])
+def test_more_batches_than_the_capacity_are_reported(ctx, n):
+    """Targets that fill a volume occupy 8^4 cells of the finest batch level, where the capacity is made for the cells
+    that a sphere meets: LPM_ERR_CAPACITY, with no more batches in use than the arrays hold (one launch cuts the batches
+    up to 131,072 targets, several above).  The level below fits, and the solver evaluates on it."""
+    torch = ctx.use_torch_stream()
+    rng = np.random.default_rng(n)
+    tgt = torch.tensor(rng.uniform(-1, 1, (n, 4)), device="cuda")
+    src = tgt[:1000].clone()
+    ts = L.TreeSum(ctx, L.biot_savart_kernel(), L.tree_solver(L.LPM_PREC_F32, 4, 64, 0.5), 1000, n)
+    ts.set_param("root_maxr", 1.0)
+    assert ts.get_param("batch_level_max") == 4 and ts.get_param("batch_cap") < 8 ** 4
+    out = torch.empty((3, n), dtype=torch.float64, device="cuda")
+    ts.set_param("batch_level", 4)
+    for _ in range(2):
+        with pytest.raises(L.LpmError, match="4096 target batches") as e:
+            ts.eval(src, tgt, out)
+        assert e.value.code == L._capi.LPM_ERR_CAPACITY
+        assert ts.stats()["batches"] == ts.get_param("batch_cap")
+    ts.set_param("batch_level", 3)
+    ts.eval(src, tgt, out)
+    assert ts.stats()["batches"] < ts.get_param("batch_cap")
+    ts.close()
