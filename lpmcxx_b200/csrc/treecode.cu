@@ -3508,8 +3508,14 @@ int tree_velocity(TreeSolver* t, const double4* src, int64_t n_src, const double
     if (cap != cudaStreamCaptureStatusNone) return tree_enqueue(t, src, n_src, X, n_tgt, U, false);
     // The first evaluation sizes the buffers as it goes (two waits of the host).  Later ones run through on the
     // buffers there are, one wait at the end, and an evaluation whose flags show an overflow is repeated with the
-    // waits: the buffers grow and every output is written again.  (50,021-point Poisson: 501 -> 439 us.)
-    for (bool careful = !t->sized;; careful = true) {
+    // waits: the buffers grow and every output is written again.  (50,021-point Poisson: 501 -> 439 us.)  Inputs that the
+    // output lies over could not be read a second time, so their evaluations wait as the first one.
+    auto under_output = [&](const double4* in, int64_t n) {
+        const char *a = (const char*)in, *b = (const char*)(in + n);
+        const char *u = (const char*)U, *v = (const char*)(U + (t->scalar ? 1 : 3) * n_tgt);
+        return a < v && u < b;
+    };
+    for (bool careful = !t->sized || under_output(src, n_src) || under_output(X, n_tgt);; careful = true) {
         int rc = tree_enqueue(t, src, n_src, X, n_tgt, U, careful);
         if (rc) t->sized = false;  // a regrow may have failed
         if (rc || n_src == 0 || n_tgt == 0) return rc;

@@ -172,3 +172,29 @@ def test_more_batches_than_the_capacity_are_reported(ctx, n):
     ts.eval(src, tgt, out)
     assert ts.stats()["batches"] < ts.get_param("batch_cap")
     ts.close()
+
+
+@pytest.mark.gpu
+def test_output_over_the_targets_survives_a_regrow(ctx):
+    """out may lie over the targets' storage (they are read before it is written), also where the evaluation needs larger
+    buffers than an earlier one left: it is then not repeated on inputs that its first pass has overwritten."""
+    torch = ctx.use_torch_stream()
+    _, p, n_src = W.gaussian_vortex_mesh("icos", 5)
+    tiny = p.copy()
+    x0 = np.array([0.0, 0.0, 1.0])
+    tiny[:, :3] = x0 + 1e-9 * (p[:, :3] - x0)
+    tiny[:, :3] /= np.linalg.norm(tiny[:, :3], axis=1, keepdims=True)
+    n = p.shape[0]
+    small, d = torch.tensor(tiny, device="cuda"), torch.tensor(p, device="cuda")
+    src, want = d[:n_src].clone(), torch.empty((3, n), dtype=torch.float64, device="cuda")
+    results = []
+    for alias in (False, True):
+        ts = L.TreeSum(ctx, L.biot_savart_kernel(), L.tree_solver(L.LPM_PREC_F32, 4, 1, 0.3), n_src, n)
+        ts.eval(small[:n_src], small, want)
+        held = ts.get_param("near_cap")
+        out = d.view(-1)[: 3 * n].view(3, n) if alias else want
+        ts.eval(src, d, out)
+        assert ts.get_param("near_cap") > held
+        results.append(out.clone())
+        ts.close()
+    assert torch.equal(*results)
