@@ -94,6 +94,15 @@ void* pinned(lpm_ctx* ctx, size_t bytes) {
     return ctx->pinned;
 }
 
+int32_t* host_state(lpm_ctx* ctx) {
+    if (!ctx->host_state && cudaMallocHost((void**)&ctx->host_state, kHostStateInts * sizeof(int32_t)) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->host_state = nullptr;
+        set_error("pinned host allocation of %zu bytes failed", kHostStateInts * sizeof(int32_t));
+    }
+    return ctx->host_state;
+}
+
 void prof_begin(lpm_ctx* ctx, LpmProfRecord& r) {
     if (cudaEventCreate(&r.start) != cudaSuccess || cudaEventCreate(&r.stop) != cudaSuccess) {
         cudaGetLastError();
@@ -222,6 +231,7 @@ int lpm_ctx_destroy(lpm_ctx* ctx) {
     for (auto& b : ctx->buf)
         if (b.ptr) cudaFree(b.ptr);
     if (ctx->pinned) cudaFreeHost(ctx->pinned);
+    if (ctx->host_state) cudaFreeHost(ctx->host_state);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     delete ctx;
     return LPM_OK;

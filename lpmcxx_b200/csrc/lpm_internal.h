@@ -48,6 +48,7 @@ struct lpm_ctx {
     // pinned host staging (host-facing entry points)
     void* pinned = nullptr;
     size_t pinned_bytes = 0;
+    int32_t* host_state = nullptr;  // pinned, kHostStateInts: what the tree solvers read back (host_state())
     // incremented whenever a scratch slot is reallocated: a CUDA graph captured before holds the old address
     uint64_t generation = 0;
     // FP32 direct sums: targets per thread of the tile kernels (2, 4 or 8; lpm_ctx_set_param "direct_targets")
@@ -94,6 +95,10 @@ enum ScratchSlot {
 // on allocation failure.
 void* scratch(lpm_ctx* ctx, int slot, size_t bytes);
 void* pinned(lpm_ctx* ctx, size_t bytes);
+// kHostStateInts pinned values for a solver's read-back, the context's one block of them (made on first use; nullptr and
+// the error set on failure): what was copied there is used up before another call on the context.
+constexpr int kHostStateInts = 64;
+int32_t* host_state(lpm_ctx* ctx);
 
 int cuda_status(cudaError_t e, const char* what);
 // cudaMalloc through the library's allocation-failure injection point (lpm_debug_fail_allocations).

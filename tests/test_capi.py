@@ -47,3 +47,11 @@ def test_no_device_is_a_status_not_a_crash():
 def test_null_context_rejected():
     k = _capi.KernelDesc(_capi.LPM_KERNEL_BIOT_SAVART_SPHERE, 0, 1.0, 0.0)
     assert _capi.lib().lpm_direct_sum_dev(None, C.byref(k), 0, None, 0, None, 0, 0, None) == _capi.LPM_ERR_ARG
+
+
+def test_pinned_host_memory_belongs_to_the_context():
+    """Pinned blocks are made once per context: an allocation of one takes milliseconds where the driver has no such page
+    left over, so a solver or tree that makes its own pays that on every creation."""
+    csrc = ROOT / "lpmcxx_b200" / "csrc"
+    users = {p.name for p in csrc.iterdir() if any(f in p.read_text() for f in ("cudaMallocHost", "cudaHostAlloc"))}
+    assert users == {"context.cu"}
