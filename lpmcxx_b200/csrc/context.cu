@@ -218,6 +218,13 @@ int lpm_ctx_create(int device, lpm_ctx** out) {
         return lpm::cuda_status(e, "cudaStreamCreate");
     }
     c->stream = c->own_stream;
+    // A small buffer that stays: the driver serves small allocations from a 2 MB chunk and gives it back with the last of
+    // them, so a context that holds none pays for the chunk in every call that allocates a little and frees it (an octree
+    // of 1,000 points 320 -> 900 us, a solver of 300 particles 0.26 -> 0.87 ms to create and 0.27 -> 0.76 to destroy).
+    if (!lpm::scratch(c, lpm::kSlotMisc2, 0)) {
+        lpm_ctx_destroy(c);
+        return LPM_ERR_OOM;
+    }
     *out = c;
     return LPM_OK;
 }

@@ -1,5 +1,9 @@
 """Octree: leaf membership and node structure bit-exact against the reference's TreeSum trees
 (golden fixtures made by the unmodified reference); the oracle on CPU, the CUDA build on GPU."""
+import subprocess
+import sys
+from pathlib import Path
+
 import numpy as np
 import pytest
 
@@ -210,3 +214,28 @@ def test_gpu_sakajo_tree_matches_reference(ctx, kind, level, depth):
     assert np.array_equal(members, g["leaf_members"])
     tree.close()
     ts.close()
+
+
+@pytest.mark.gpu
+def test_small_buffers_come_from_a_chunk_the_context_keeps():
+    """The driver serves small allocations from a chunk that it gives back with the last of them.  A context holds one
+    buffer from its creation on, so building and dropping a small tree (all its arrays are small) maps no memory."""
+    prog = '''
+import torch, lpmcxx_b200 as L
+ctx = L.Context(0)
+torch.cuda.init()
+pts = torch.rand((1000, 4), dtype=torch.float64, device="cuda") * 2 - 1
+ctx.use_torch_stream()
+free = []
+for _ in range(3):
+    tree = L.Tree(ctx, pts, (-1.0, 1.0) * 3, 40, 10)
+    torch.cuda.synchronize()
+    free.append(torch.cuda.mem_get_info()[0])
+    tree.close()
+    free.append(torch.cuda.mem_get_info()[0])
+print(len(set(free[2:])))
+'''
+    out = subprocess.run([sys.executable, "-c", prog], capture_output=True, text=True, timeout=300,
+                         cwd=Path(__file__).resolve().parent.parent)
+    assert out.returncode == 0, out.stderr
+    assert out.stdout.split()[-1] == "1"
