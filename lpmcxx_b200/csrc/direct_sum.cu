@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(kThreads64, 4) direct64_kernel(const double4* 
 #pragma unroll
     for (int t = 0; t < TPT; ++t) {
         const int64_t i = blk0 + lt + t * gw;
-        const double4 p = i < n_tgt ? tgt[i] : make_double4(0.0, 0.0, 2.0, 0.0);
+        const double4 p = i < n_tgt ? tgt[i] : make_double4(0.0, 0.0, 0.0, 0.0);  // den R^2: never a close pair
         tx[t] = p.x; ty[t] = p.y; tz[t] = p.z;
         odd = odd || odd_point(p);
         self[t] = Op::kSelf && i < coinc_n ? coinc_off + i : -1;

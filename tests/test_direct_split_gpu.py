@@ -134,3 +134,17 @@ def test_log_kernels_to_the_last_bits(ctx, kernel, scale):
         ref = np.log(z) / (4 * np.longdouble(np.pi))
     tol = 2.0 ** -53 * (2 * (2 * np.abs(np.log(z)) + 0.7) + cond) / (4 * np.pi)
     assert np.max(np.abs(got - ref) / tol) < 1.0
+
+
+@pytest.mark.parametrize("kernel,comps", [(L.biot_savart_kernel(), 3), (L.biot_savart_kernel(1.0, 0.03), 3),
+                                          (L.sphere_greens_kernel(), 1), (L.poisson_kernel(), 1)])
+def test_targets_missing_from_a_block_change_nothing(ctx, kernel, comps):
+    """Targets far from every source (none takes the path of close pairs) have the same sums, bit for bit, in a full block
+    of 64 as in one that holds only them: what stands in for missing targets sends no warp down another path."""
+    ctx.use_torch_stream()
+    x = random_sphere(3000, 3)
+    north, south = x[x[:, 2] > 0.3][:700], x[x[:, 2] < -0.2][:64]
+    src, tgt = oracle.pack4(north, np.linspace(-1.0, 1.0, 700)), oracle.pack4(south)
+    full = _sum(ctx, kernel, L.LPM_PREC_F64, src, tgt, comps, 0)
+    for n in (1, 2, 33, 63):
+        assert np.array_equal(_sum(ctx, kernel, L.LPM_PREC_F64, src, tgt[:n], comps, 0), full[:, :n]), n
