@@ -166,6 +166,7 @@ template <bool kDelta, int kTPT>
 struct BsF64 {
     static constexpr int NC = 3, TPT = kTPT;
     static constexpr bool kSelf = false, kAux = true, kCheck = true;
+    static constexpr int kCrowd = 5;
     double r2, d2, c0;   // R^2, delta^2, R^2 + delta^2
     int lo;              // a den whose high word is at least lo takes the common path
 
@@ -255,6 +256,7 @@ template <int kTPT>
 struct PoissonF64 {
     static constexpr int NC = 1, TPT = kTPT;
     static constexpr bool kSelf = false, kAux = false, kCheck = true;
+    static constexpr int kCrowd = 5;
 
     __device__ __forceinline__ static NoState init() { return NoState{}; }
     __device__ __forceinline__ static double4 prepare(const double4& y) { return y; }
@@ -324,6 +326,7 @@ template <class K>
 struct ScalarF64 {
     static constexpr int NC = 1, TPT = 2;
     static constexpr bool kSelf = false, kAux = false, kCheck = false;
+    static constexpr int kCrowd = 24;
     K kern;
 
     __device__ __forceinline__ static NoState init() { return NoState{}; }
@@ -381,6 +384,7 @@ template <class Arg>
 struct LogF64 {
     static constexpr int NC = 2, TPT = 2;  // sum w (log z - k log 2), sum w k
     static constexpr bool kSelf = true, kAux = false, kCheck = true;
+    static constexpr int kCrowd = 24;
     Arg arg;
 
     struct State {  // the lane's entry of the table: the high word of c, -log c
@@ -539,6 +543,48 @@ __global__ void __launch_bounds__(kThreads64, 4) direct64_kernel(const double4* 
     reduce_split<TPT, NC, kThreads64>(totals, sp, rank, [&](int u, const double (&v)[NC]) {
         if (blk0 + u < n_tgt) op.finish(blk0 + u, v, tgt, mult, out, stride);
     });
+}
+
+// FP64 direct sum of at most kFew sources: one per thread to stage, no groups, parts or totals; a thread sums its targets
+// over all of them and writes its results.  Bound by the targets' loads and the results' stores: at few sources the
+// totals' way through shared memory costs more than the pairs (1 source x 300,000 / 1M targets 14.7 / 41 us by
+// direct64_kernel in four groups, 10.6 / 27 in one).
+constexpr int kFew = kThreads64;
+template <class Op>
+__global__ void __launch_bounds__(kThreads64) direct64_few_kernel(const double4* __restrict__ src, int n_src,
+                                                                  const double4* __restrict__ tgt, int64_t n_tgt, Op op,
+                                                                  double mult, double* __restrict__ out, int64_t stride,
+                                                                  int64_t coinc_n, int64_t coinc_off) {
+    constexpr int TPT = Op::TPT, NC = Op::NC;
+    __shared__ double4 st[Op::kAux ? 2 * kFew : kFew];
+    const int64_t first = (int64_t)blockIdx.x * (kThreads64 * TPT) + threadIdx.x;
+    double tx[TPT], ty[TPT], tz[TPT], s[TPT][NC];
+    int64_t self[TPT];
+    bool odd = false, bad = false;
+#pragma unroll
+    for (int t = 0; t < TPT; ++t) {
+        const int64_t i = first + t * kThreads64;
+        const double4 p = i < n_tgt ? tgt[i] : make_double4(0.0, 0.0, 0.0, 0.0);  // as in direct64_kernel
+        tx[t] = p.x; ty[t] = p.y; tz[t] = p.z;
+        odd = odd || odd_point(p);
+        self[t] = Op::kSelf && i < coinc_n ? coinc_off + i : -1;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) s[t][c] = 0.0;
+    }
+    if ((int)threadIdx.x < n_src) {
+        const double4 y = src[threadIdx.x];
+        st[threadIdx.x] = y;
+        bad = odd_point(y) || odd_strength(y.w);
+        if constexpr (Op::kAux) st[kFew + threadIdx.x] = Op::prepare(y);
+    }
+    const auto state = op.init();
+    const bool plain = !__syncthreads_or(bad) && !__any_sync(0xffffffffu, odd);
+    op.tile(state, st, st + kFew, n_src, plain, 0, tx, ty, tz, self, s);
+#pragma unroll
+    for (int t = 0; t < TPT; ++t) {
+        const int64_t i = first + t * kThreads64;
+        if (i < n_tgt) op.finish(i, s[t], tgt, mult, out, stride);
+    }
 }
 
 // ------------------------------------------------------------------ FP32 Biot-Savart
@@ -726,19 +772,30 @@ int pack_f32(lpm_ctx* ctx, const double4* in, int64_t n, float4* out, bool scale
 }
 
 namespace {
-// Splits of a direct sum of n_tgt targets.  FP64: four groups per block at every size (more blocks of fewer targets
-// fill the last wave better; 81,920 sources: 12.3 ms with one group and part, 8.6 ms with four groups and two parts),
-// and eight parts while the blocks alone are fewer than the four resident per SM, two above (1,280 / 20,480 sources:
-// 16.8 / 602 us with eight parts, 27.1 / 752 us with two; 81,920: 8.80 ms with eight, 8.64 ms with two).  A warp keeps
-// at least 16 sources.
+// Splits of a direct sum of n_tgt targets.  FP64: four groups per block at every size (more blocks of fewer targets fill
+// the last wave better; 81,920 sources x 122,882 targets took 1.4 times as long with one group and part), and eight parts
+// while the blocks alone are fewer than the four resident per SM, two above (1,280 sources x 1,922 targets / 20,480 x
+// 30,722: 12.3 / 525 us with eight parts, two cost a third more).  A part keeps at least 64 sources (a warp 16), and 256
+// where blocks x parts are more than Op::kCrowd per SM: a block's fixed cost (targets, totals, the sums' reduction) then
+// outweighs a short run of sources.  75,000 targets, Biot-Savart, 130 / 257 / 700 / 1,000 sources: 16.7 / 27 / 56 / 76 us so
+// and 20.8 / 40 / 97 / 111 us with 64 everywhere; the scalar kernels, with fewer targets a block and longer pairs, gain
+// from parts up to 16 blocks per SM (Green's function, 40,000 targets, 400 sources: 41 us with two parts, 51 with one) and
+// lose beyond (300,000 targets, 130 sources: 107 and 84).
 int64_t blocks64(int64_t n_tgt, int tpt) {
     const int64_t tb = (kThreads64 * tpt) >> 2;
     return (n_tgt + tb - 1) / tb;
 }
-Split split64(int sms, int64_t blocks, int64_t n_src) {
+Split split64(int sms, int64_t blocks, int64_t n_src, int crowd) {
     int parts = blocks < 4 * (int64_t)sms ? 8 : 2;
-    while (parts > 1 && n_src < 64 * parts) parts /= 2;
+    while (parts > 1 && n_src < (int64_t)parts * (blocks * parts > crowd * (int64_t)sms ? 256 : 64)) parts /= 2;
     return Split{2, parts};
+}
+
+// Whether a sum goes to direct64_few_kernel, which has a quarter of direct64_kernel's blocks: by targets per SM.  1 / 8 / 30
+// / 128 sources by either (Biot-Savart, us): 75,000 targets 5.0 / 5.1 / 9.0 / 20.8 against 6.0 / 6.5 / 8.5 / 16.7, 150,000
+// 5.5 / 5.9 / 10.5 / 24.9 against 9.0 / 10.5 / 12.7 / 25.3, 1M 10.5 / 18.8 / 35.2 / 119 against 41 / 47 / 62 / 135.
+bool few_sources(int sms, int64_t n_tgt, int64_t n_src) {
+    return n_src <= kFew && n_tgt >= sms * std::min<int64_t>(1000, 100 + 40 * n_src);
 }
 
 // FP32: the estimated time of `rounds` of stages (one tile per group) at the blocks each SM holds, in units fitted to
@@ -777,11 +834,15 @@ bool few_targets(const lpm_ctx* ctx, int64_t n_tgt) { return blocks64(n_tgt, 4) 
 template <class Op>
 int launch64(lpm_ctx* ctx, const char* name, Op op, const double4* src, int64_t n_src, const double4* tgt,
              int64_t n_tgt, double mult, double* out, int64_t stride, int64_t coinc_n, int64_t coinc_off) {
+    if (few_sources(ctx->num_sms, n_tgt, n_src)) {
+        LPM_LAUNCH(ctx, name, direct64_few_kernel<Op>, grid_for(n_tgt, kThreads64 * Op::TPT), kThreads64, 0, src, (int)n_src,
+                   tgt, n_tgt, op, mult, out, stride, coinc_n, coinc_off);
+        return LPM_OK;
+    }
     const int64_t blocks = blocks64(n_tgt, Op::TPT);
-    const Split sp = split64(ctx->num_sms, blocks, n_src);
+    const Split sp = split64(ctx->num_sms, blocks, n_src, Op::kCrowd);
     const size_t smem = Shape64<Op>::kSmem;
-    if (smem > 48 * 1024)
-        LPM_CUDA_TRY(cudaFuncSetAttribute(direct64_kernel<Op>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    static_assert(Shape64<Op>::kSmem <= 48 * 1024, "no opt-in needed");
     return launch_cluster(ctx, name, direct64_kernel<Op>, (unsigned)(blocks * sp.parts), kThreads64, smem, sp.parts, src,
                           n_src, tgt, n_tgt, op, mult, out, stride, coinc_n, coinc_off, sp);
 }

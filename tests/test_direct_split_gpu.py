@@ -148,3 +148,30 @@ def test_targets_missing_from_a_block_change_nothing(ctx, kernel, comps):
     full = _sum(ctx, kernel, L.LPM_PREC_F64, src, tgt, comps, 0)
     for n in (1, 2, 33, 63):
         assert np.array_equal(_sum(ctx, kernel, L.LPM_PREC_F64, src, tgt[:n], comps, 0), full[:, :n]), n
+
+
+@pytest.mark.parametrize("n_src,n_tgt", [(0, 20721), (1, 20719), (1, 20721), (2, 30001), (127, 147999), (128, 148001),
+                                         (129, 148001), (257, 75003), (511, 75003), (513, 113667), (1025, 75003)])
+@pytest.mark.parametrize("name", ["bs", "bs_delta", "poisson", "greens", "log", "delta3d", "sphere_delta"])
+def test_few_sources_many_targets(ctx, name, n_src, n_tgt):
+    """Around the targets per SM from which up to 128 sources take the kernel without splits, and around the sources from
+    which crowded SMs get parts; the reference on the first, the last and every 37th target."""
+    ctx.use_torch_stream()
+    make, kind, param = {"bs": (L.biot_savart_kernel, 1, 0.0), "bs_delta": (L.biot_savart_kernel, 1, 0.03),
+                         "poisson": (L.poisson_kernel, 2, 0.0), "greens": (L.sphere_greens_kernel, 3, 1.0),
+                         "log": (L.planar_log_kernel, 4, 0.0), "delta3d": (L.delta3d_kernel, 5, 0.2),
+                         "sphere_delta": (L.sphere_delta_kernel, 6, 0.2)}[name]
+    kernel = make(1.0, param) if kind == 1 else make(param) if kind in (3, 5, 6) else make()
+    src, tgt = _data(n_src, n_tgt, name in ("poisson", "log", "delta3d"))
+    pick = np.unique(np.r_[:min(300, n_tgt), 0:n_tgt:37, n_tgt - 300:n_tgt])
+    own = np.where(pick < n_src, pick, -1)
+    got = _sum(ctx, kernel, L.LPM_PREC_F64, src, tgt, 3 if kind == 1 else 1, n_src)[:, pick]
+    if n_src == 0:
+        assert not got.any()
+    elif kind == 1:
+        assert rel_linf(got, oracle.bs_direct(src, tgt[pick], delta=param)) < 1e-12
+    elif kind == 2:
+        assert rel_linf(got[0], oracle.poisson_direct(src, tgt[pick])) < 1e-12
+    else:
+        ref = oracle.scalar_direct(kind, param, src, tgt[pick], own if kind in (3, 4) else None)
+        assert rel_linf(got[0], ref) < 1e-12
