@@ -774,8 +774,8 @@ int pack_f32(lpm_ctx* ctx, const double4* in, int64_t n, float4* out, bool scale
 namespace {
 // Splits of a direct sum of n_tgt targets.  FP64: four groups per block at every size (more blocks of fewer targets fill
 // the last wave better; 81,920 sources x 122,882 targets took 1.4 times as long with one group and part), and eight parts
-// while the blocks alone are fewer than the four resident per SM, two above (1,280 sources x 1,922 targets / 20,480 x
-// 30,722: 12.3 / 525 us with eight parts, two cost a third more).  A part keeps at least 64 sources (a warp 16), and 256
+// while the blocks alone are fewer than the four resident per SM, two above (1,500 sources x 5,000 targets / 16,000 x 20,000
+// 22 / 312 us with eight parts, 31 / 433 with two; 16,000 x 150,000 2.10 ms with eight, 2.02 with two).  A part keeps at least 64 sources (a warp 16), and 256
 // where blocks x parts are more than Op::kCrowd per SM: a block's fixed cost (targets, totals, the sums' reduction) then
 // outweighs a short run of sources.  75,000 targets, Biot-Savart, 130 / 257 / 700 / 1,000 sources: 16.7 / 27 / 56 / 76 us so
 // and 20.8 / 40 / 97 / 111 us with 64 everywhere; the scalar kernels, with fewer targets a block and longer pairs, gain
@@ -800,29 +800,41 @@ bool few_sources(int sms, int64_t n_tgt, int64_t n_src) {
 
 // FP32: the estimated time of `rounds` of stages (one tile per group) at the blocks each SM holds, in units fitted to
 // 640 ... 327,680 sources (a round takes 19 / 30 / 55 us with 1 / 2 / 4 blocks of 256 x 4 targets on the SM); clusters
-// of four and eight blocks lose 15% and 30% where the blocks are many times the resident ones.
+// of four and eight blocks lose 15% and 30% where the blocks are many times the resident ones.  Few tiles on many
+// targets share out badly: groups that have none hold their block's place on the SM while the others work, so there fewer
+// groups count too, a round of the last tile alone as long as that tile is, and a round's time by how full its groups
+// are.  Biot-Savart, 257 / 700 / 1,100 / 1,300 sources x 1M targets 134 / 292 / 504 / 599 us with four groups and two parts
+// from three and five tiles on, 112 / 274 / 416 / 495 so; 1,000 sources (four tiles) 368 us with four groups, 383 with one.
 struct Split32 {
     int tpt;
     Split split;
 };
 Split32 split32(int sms, int64_t n_tgt, int64_t n_src, int max_tpt) {
     const int64_t tiles = std::max<int64_t>(1, (n_src + kTile - 1) / kTile);
-    const int gs = tiles >= 3 ? 2 : (tiles == 2 ? 1 : 0);
-    Split32 best{max_tpt, Split{gs, 1}};
+    const double last = (double)(n_src - (tiles - 1) * kTile) / kTile;
+    const bool uneven = tiles <= 8 && n_tgt >= 1000 * (int64_t)sms;
+    const int most = tiles >= 3 ? 2 : (tiles == 2 ? 1 : 0);
+    Split32 best{max_tpt, Split{most, 1}};
     double best_cost = 0.0;
     for (int tpt = max_tpt; tpt >= 2; tpt /= 2)
-        for (int parts = 1; parts <= 8 && parts <= tiles; parts *= 2) {
-            const int64_t per_part = (tiles + parts - 1) / parts, tb = (kThreads * tpt) >> gs;
-            const int64_t blocks = (n_tgt + tb - 1) / tb * parts;
-            if (tpt < max_tpt && blocks > 2 * (int64_t)sms) break;  // fewer targets per thread read more per pair
-            const double rounds = (double)((per_part + (1 << gs) - 1) >> gs);
-            const double loss = blocks > 4 * (int64_t)sms && parts > 2 ? (parts == 8 ? 1.3 : 1.15) : 1.0;
-            const double cost = loss * rounds * tpt * (7.0 + 12.0 * std::ceil((double)blocks / std::max(sms, 1)));
-            if ((tpt == max_tpt && parts == 1) || cost < 0.985 * best_cost) {
-                best = Split32{tpt, Split{gs, parts}};
-                best_cost = cost;
+        for (int gs = most; gs >= (uneven ? 0 : most); --gs)
+            for (int parts = 1; parts <= 8 && parts <= tiles; parts *= 2) {
+                const int64_t per_part = (tiles + parts - 1) / parts, tb = (kThreads * tpt) >> gs;
+                const int64_t blocks = (n_tgt + tb - 1) / tb * parts;
+                if (tpt < max_tpt && blocks > 2 * (int64_t)sms) break;  // fewer targets per thread read more per pair
+                double rounds = (double)((per_part + (1 << gs) - 1) >> gs), fill = 1.0;
+                if (uneven && parts == 1) {
+                    if (((tiles - 1) & ((1 << gs) - 1)) == 0) rounds += last - 1.0;
+                    fill = (double)n_src / std::max(1.0, rounds * (kTile << gs));
+                }
+                const double loss = blocks > 4 * (int64_t)sms && parts > 2 ? (parts == 8 ? 1.3 : 1.15) : 1.0;
+                const double cost = loss * rounds * tpt *
+                                    (7.0 + (3.0 + 9.0 * fill) * std::ceil((double)blocks / std::max(sms, 1)));
+                if ((tpt == max_tpt && gs == most && parts == 1) || cost < 0.985 * best_cost) {
+                    best = Split32{tpt, Split{gs, parts}};
+                    best_cost = cost;
+                }
             }
-        }
     return best;
 }
 

@@ -175,3 +175,18 @@ def test_few_sources_many_targets(ctx, name, n_src, n_tgt):
     else:
         ref = oracle.scalar_direct(kind, param, src, tgt[pick], own if kind in (3, 4) else None)
         assert rel_linf(got[0], ref) < 1e-12
+
+
+@pytest.mark.parametrize("n_src,n_tgt", [(1, 148001), (256, 148001), (257, 147999), (257, 148001), (700, 300001),
+                                         (1100, 300001), (2048, 148001), (2049, 148001)])
+@pytest.mark.parametrize("scalar", [False, True])
+def test_few_tiles_many_targets_f32(ctx, n_src, n_tgt, scalar):
+    """Around the tiles and the targets per SM from which fewer groups share the tiles; the reference on the first, the
+    last and every 37th target."""
+    ctx.use_torch_stream()
+    kernel = L.poisson_kernel() if scalar else L.biot_savart_kernel()
+    src, tgt = _data(n_src, n_tgt, scalar)
+    pick = np.unique(np.r_[:300, 0:n_tgt:37, n_tgt - 300:n_tgt])
+    got = _sum(ctx, kernel, L.LPM_PREC_F32, src, tgt, 1 if scalar else 3, n_src)[:, pick]
+    ref = oracle.poisson_direct(src, tgt[pick])[None] if scalar else oracle.bs_direct(src, tgt[pick])
+    assert rel_l2(got, ref) < 5e-6
