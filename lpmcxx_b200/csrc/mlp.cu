@@ -166,19 +166,25 @@ __global__ void mlp_to_bf16_kernel(const float* __restrict__ params, __nv_bfloat
     if (p < kMlpParams) w[p] = __float2bfloat16_rn(params[p]);
 }
 
-// The treecode's inference path (mlp_warp_argmax): 32 samples per warp on the tensor cores.
+// The treecode's inference path (mlp_warp_argmax): 32 samples per warp on the tensor cores, on weights staged once a block
+// as the traversal's (read from global memory, twice for the two tiles of 16 rows, 500,000 samples took 108 us; so 73).
 __global__ void __launch_bounds__(128) mlp_predict_bf16_kernel(const __nv_bfloat16* __restrict__ w,
                                                                const float* __restrict__ norm,
                                                                const float* __restrict__ feats, int64_t n,
                                                                int32_t* __restrict__ cls) {
+    __shared__ __align__(16) __nv_bfloat16 sw[MlpLayout<kMlpPad>::kSize];
     __shared__ __align__(16) __nv_bfloat16 xs[4][32 * kMlpIn];
-    const int64_t base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31);
-    if (base >= n) return;  // uniform per warp
-    const int64_t i = base + (threadIdx.x & 31);
-    float f[kMlpIn];
-    for (int k = 0; k < kMlpIn; ++k) f[k] = i < n ? feats[i * kMlpIn + k] : norm[k];
-    const int c = mlp_warp_argmax<0>(w, norm, f, xs[threadIdx.x >> 5], threadIdx.x & 31, (int)min((int64_t)32, n - base));
-    if (i < n) cls[i] = c;
+    mlp_stage<kMlpPad>(w, sw);
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    for (int64_t base = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; base < n;
+         base += (int64_t)gridDim.x * blockDim.x) {  // uniform per warp
+        const int64_t i = base + lane;
+        float f[kMlpIn];
+        for (int k = 0; k < kMlpIn; ++k) f[k] = i < n ? feats[i * kMlpIn + k] : norm[k];
+        const int c = mlp_warp_argmax<kMlpPad>(sw, norm, f, xs[threadIdx.x >> 5], lane, (int)min((int64_t)32, n - base));
+        if (i < n) cls[i] = c;
+    }
 }
 
 int train_smem_bytes() { return kTrainSmemFloats * (int)sizeof(float); }
@@ -330,7 +336,8 @@ extern "C" int lpm_mlp_predict(lpm_ctx* ctx, const float* params, const float* f
     int rc = mlp_upload_bf16(ctx, params, (__nv_bfloat16*)bw.p, (float*)bn.p);
     if (rc) return rc;
     LPM_CUDA_TRY(cudaMemcpyAsync(bf.p, feats, (size_t)n * kMlpIn * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
-    LPM_LAUNCH(ctx, "mlp_predict_bf16_kernel", mlp_predict_bf16_kernel, grid_for(n, 128), 128, 0,
+    const unsigned blocks = std::min<unsigned>(grid_for(n, 128), 4 * (unsigned)ctx->num_sms);
+    LPM_LAUNCH(ctx, "mlp_predict_bf16_kernel", mlp_predict_bf16_kernel, blocks, 128, 0,
                (const __nv_bfloat16*)bw.p, (const float*)bn.p, (const float*)bf.p, n, (int32_t*)bc.p);
     LPM_CUDA_TRY(cudaMemcpyAsync(classes, bc.p, (size_t)n * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
     LPM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));

@@ -62,6 +62,7 @@ struct MlpLayout {
     static constexpr int kB2 = kW2 + kMlpHidden * kRow, kW3 = kB2 + kMlpHidden, kB3 = kW3 + kMlpOut * kRow;
     static constexpr int kSize = (kB3 + kMlpOut + 7) / 8 * 8;
 };
+constexpr int kMlpPad = 8;
 // the layout of global memory (16-byte aligned, kMlpParams values), copied to the one with kPad in shared memory by the
 // whole block, 8 values at a time: every array but the last begins and ends on a multiple of 8 (no barrier)
 template <int kPad>

@@ -578,7 +578,6 @@ struct TraverseArgs {
 
 constexpr int kWarpStack = 1024;
 constexpr int kDecisionCap = 1024;  // cached selector decisions per batch
-constexpr int kMlpPad = 8;             // MlpLayout of the selector's weights in shared memory
 constexpr int kOrderBits = 4;         // an order fits
 static_assert(kPMax < 1 << kOrderBits, "orders are told apart by kOrderBits ballots");
 

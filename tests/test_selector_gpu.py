@@ -43,3 +43,14 @@ def test_classes_at_tile_edges(ctx, n):
     params = learned.load()[0]
     f = np.random.default_rng(5).normal(size=(1024, 8)).astype(np.float32) * 2.0
     assert np.array_equal(L.mlp_predict(ctx, params, f[:n]), L.mlp_predict(ctx, params, f)[:n])
+
+
+@pytest.mark.parametrize("n", [1, 127, 129, 75775, 75777, 151553])
+def test_predictions_do_not_depend_on_the_grid(ctx, n):
+    """One launch of at most four blocks per SM, whose warps take 32 samples at a time: the classes of n samples are those
+    of their runs of 1,000 samples (no warp takes more than 32 there)."""
+    params = learned.load()[0]
+    feats = np.random.default_rng(n).normal(size=(n, 8)).astype(np.float32)
+    got = L.mlp_predict(ctx, params, feats)
+    runs = [L.mlp_predict(ctx, params, feats[i:i + 1000]) for i in range(0, n, 1000)]
+    assert np.array_equal(got, np.concatenate(runs))
