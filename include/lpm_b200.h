@@ -269,7 +269,7 @@ int lpm_treesum_create(lpm_ctx* ctx, const lpm_kernel_desc* kernel, const lpm_so
                        int64_t n_tgt, lpm_treesum** out);
 int lpm_treesum_destroy(lpm_treesum* ts);
 /* Device arrays: src n_src x 4 (x,y,z,w), tgt n_tgt x 4, out 3 x n_tgt (component-major; Poisson:
- * 1 x n_tgt).  Replaces TreeSum::computeMeshMoments + meshSolve (src/LpmTreeSum.cpp:55-86,182-197) for
+ * 1 x n_tgt; it may lie over src or tgt).  Replaces TreeSum::computeMeshMoments + meshSolve (src/LpmTreeSum.cpp:55-86,182-197) for
  * device-resident data. */
 int lpm_treesum_eval_dev(lpm_treesum* ts, const double* src, const double* tgt, double* out);
 /* Statistics of the last evaluation, 10 values: nodes, leaves, depth, far (batch, cluster) pairs, near
@@ -297,7 +297,9 @@ int lpm_treesum_stats(lpm_treesum* ts, int64_t* out10);
  * evaluation fail with LPM_ERR_ARG.  Parameters take effect at the next evaluation. */
 int lpm_treesum_set_param(lpm_treesum* ts, const char* name, double value);
 /* Current value of a run-time parameter: those of lpm_treesum_set_param, plus "batch_level_max" (the finest
- * batch level allowed) and "order" (the fixed order in the solver's convention: Poisson reports p + 1). */
+ * batch level allowed), "order" (the fixed order in the solver's convention: Poisson reports p + 1) and what the
+ * solver's buffers hold: "batch_cap" target batches, "far_cap" and "near_cap" interaction-list entries, "heavy_cap"
+ * nodes with moments (0 after a regrow that failed; the next evaluation allocates again). */
 int lpm_treesum_get_param(const lpm_treesum* ts, const char* name, double* value);
 /* The source octree of the solver's last evaluation as a read-only lpm_tree (lpm_tree_counts,
  * lpm_tree_leaf_membership and lpm_tree_nodes apply; member indices refer to the evaluation's source array):

@@ -160,8 +160,9 @@ __device__ __forceinline__ bool odd_strength(double w) {
 // next source are formed beside the current one's reciprocals and sums, so that the two chains overlap.  What bounds
 // the kernel now is the register file beside the pipe: an FP64 FMA of three distinct register operands issues every
 // three cycles instead of two (a probe of the instruction alone), and the ~9 other instructions a pair share its
-// ports.  81,920 sources x 122,882 targets: 14.26 -> 8.4 ms (12.0 -> 20.4 TFLOP/s at 17 flops a pair); two or four
-// sources a vote, two targets a thread, or more resident warps with fewer registers measured 8.3 - 10.2 ms.
+// ports.  81,920 sources x 122,882 targets: 14.26 -> 8.0 ms (12.0 -> 21.4 TFLOP/s at 17 flops a pair).  Two or four
+// sources a vote, two targets a thread, or more resident warps with fewer registers: 8.3 - 10.2 ms where this form took
+// 8.35 (with missing targets on the long path).
 template <bool kDelta, int kTPT>
 struct BsF64 {
     static constexpr int NC = 3, TPT = kTPT;
@@ -378,7 +379,7 @@ struct PlanarLogArg {
 // m = 1), log z = k log 2 - log c + log1p(r), log1p by its series to r^9 (the remainder is below 2^-57 of r).  The table is
 // one entry per lane, read by shuffles.  k log 2 is summed as sum w k and multiplied once a target.  17 FP64 operations
 // a pair; a pair with a small or not finite z, a tile that holds a target's own source and every other special case take
-// the library's log on the reference's rounding.  20,480 sources x 30,722 targets from host arrays: 2.64 -> 1.77 ms (9.17
+// the library's log on the reference's rounding.  20,480 sources x 30,722 targets from host arrays: 2.64 -> 1.6 ms (9.17
 // before the sources were split); relative L2 error against 64-bit sums 2.8e-16, as with the library's log.
 template <class Arg>
 struct LogF64 {
@@ -457,7 +458,7 @@ struct LogF64 {
 // cp.async one tile ahead of the tile being summed; the groups take consecutive shares of every tile.  A tile's sums
 // start from zero and are then added to the thread's totals, which stay in shared memory between tiles (one read and
 // write a tile).  Blocks of 128 threads: a barrier a tile holds four warps together, and the warps' times differ
-// where close pairs send some of them through the long path (against 256 threads: 8.35 against 8.8 ms on 81,920
+// where close pairs send some of them through the long path (8.35 against 8.8 ms by 256 threads on 81,920
 // sources x 122,882 targets).
 template <class Op>
 struct Shape64 {

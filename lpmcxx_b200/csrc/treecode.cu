@@ -1762,113 +1762,113 @@ __global__ void __launch_bounds__(kBatch / T) far_scalar_kernel(FarArgs A, int s
     const ClusterPart cp = kSplit ? ClusterPart{(int)(blockIdx.x % (unsigned)parts), parts} : ClusterPart{0, 1};
     if constexpr (kSplit) cluster_barrier();  // every block of the cluster runs before another touches its shared memory
     for (int round = 0;; ++round) {
-    const int64_t b = kSplit ? next_batch_split(A.ticket, A.order, nbat, slot, round, cp)
-                             : next_batch(A.ticket, A.order, nbat, slot);
-    if (b < 0) break;
-    const int64_t f0 = A.far_off[b], f1 = min(f0 + (int64_t)A.far_cnt[b], A.far_cap);
-    if (f0 >= f1) continue;  // uniform per block (and cluster)
-    const int64_t first = f0 + (int64_t)kK * cp.rank, step = (int64_t)kK * cp.parts;
-    const int64_t q0 = A.batch_first[b], qe = A.batch_first[b + 1];
-    // warp w holds targets 32 T w .. 32 T (w + 1) - 1 of the batch (lane l: 32 T w + l + 32 t), so a warp past
-    // the batch's last target idles as a whole
-    const int64_t q = q0 + 32 * T * (threadIdx.x >> 5) + (threadIdx.x & 31);
-    const bool live = q0 + 32 * T * (int64_t)(threadIdx.x >> 5) < qe;  // warp-uniform
-    // T = 2 (FP32): targets and cluster centres as FP32 offsets from the batch's first target o, so that
-    // d = c - x is one FP32 subtraction (the far2 kernel's scheme), and each stage's sums in FP32 folded into
-    // FP64 once per stage; T = 1: FP64 positions, d rounded once from the FP64 difference
-    const double4 o = A.tgt_sorted[q0];
-    double4 x[T];
-    float xo[T][3];
+        const int64_t b = kSplit ? next_batch_split(A.ticket, A.order, nbat, slot, round, cp)
+                                 : next_batch(A.ticket, A.order, nbat, slot);
+        if (b < 0) break;
+        const int64_t f0 = A.far_off[b], f1 = min(f0 + (int64_t)A.far_cnt[b], A.far_cap);
+        if (f0 >= f1) continue;  // uniform per block (and cluster)
+        const int64_t first = f0 + (int64_t)kK * cp.rank, step = (int64_t)kK * cp.parts;
+        const int64_t q0 = A.batch_first[b], qe = A.batch_first[b + 1];
+        // warp w holds targets 32 T w .. 32 T (w + 1) - 1 of the batch (lane l: 32 T w + l + 32 t), so a warp past
+        // the batch's last target idles as a whole
+        const int64_t q = q0 + 32 * T * (threadIdx.x >> 5) + (threadIdx.x & 31);
+        const bool live = q0 + 32 * T * (int64_t)(threadIdx.x >> 5) < qe;  // warp-uniform
+        // T = 2 (FP32): targets and cluster centres as FP32 offsets from the batch's first target o, so that
+        // d = c - x is one FP32 subtraction (the far2 kernel's scheme), and each stage's sums in FP32 folded into
+        // FP64 once per stage; T = 1: FP64 positions, d rounded once from the FP64 difference
+        const double4 o = A.tgt_sorted[q0];
+        double4 x[T];
+        float xo[T][3];
 #pragma unroll
-    for (int t = 0; t < T; ++t) {
-        x[t] = q + 32 * t < qe ? A.tgt_sorted[q + 32 * t] : make_double4(o.x + 4.0, o.y + 4.0, o.z + 4.0, 0);
-        xo[t][0] = (float)(x[t].x - o.x);
-        xo[t][1] = (float)(x[t].y - o.y);
-        xo[t][2] = (float)(x[t].z - o.z);
-    }
-    float4* ctrf = reinterpret_cast<float4*>(ctr);  // T = 2: 2 x kK FP32 centre offsets in the centres' space
-    const F* base = (const F*)(sizeof(F) == 8 ? (const void*)A.B64 : (const void*)A.B32);
-    auto gather = [&](int64_t s0, int n, float4* buf, int slot) {
-        for (int i = threadIdx.x; i < n * kUnits; i += kNT) {
-            const int e = i / kUnits, j = i - e * kUnits;
-            cp_async16(buf + i, (const char*)(base + (size_t)A.far_list[s0 + e].x * stride) + 16 * j);
+        for (int t = 0; t < T; ++t) {
+            x[t] = q + 32 * t < qe ? A.tgt_sorted[q + 32 * t] : make_double4(o.x + 4.0, o.y + 4.0, o.z + 4.0, 0);
+            xo[t][0] = (float)(x[t].x - o.x);
+            xo[t][1] = (float)(x[t].y - o.y);
+            xo[t][2] = (float)(x[t].z - o.z);
         }
-        if ((int)threadIdx.x < n) {
-            const double4 c = A.node_ctr[A.far_list[s0 + threadIdx.x].x];
-            if constexpr (T == 2)
-                ctrf[slot * kK + threadIdx.x] =
-                    make_float4((float)(c.x - o.x), (float)(c.y - o.y), (float)(c.z - o.z), 0.0f);
-            else
-                ctr[slot * kK + threadIdx.x] = c;
-        }
-    };
-    double acc[T];
+        float4* ctrf = reinterpret_cast<float4*>(ctr);  // T = 2: 2 x kK FP32 centre offsets in the centres' space
+        const F* base = (const F*)(sizeof(F) == 8 ? (const void*)A.B64 : (const void*)A.B32);
+        auto gather = [&](int64_t s0, int n, float4* buf, int slot) {
+            for (int i = threadIdx.x; i < n * kUnits; i += kNT) {
+                const int e = i / kUnits, j = i - e * kUnits;
+                cp_async16(buf + i, (const char*)(base + (size_t)A.far_list[s0 + e].x * stride) + 16 * j);
+            }
+            if ((int)threadIdx.x < n) {
+                const double4 c = A.node_ctr[A.far_list[s0 + threadIdx.x].x];
+                if constexpr (T == 2)
+                    ctrf[slot * kK + threadIdx.x] =
+                        make_float4((float)(c.x - o.x), (float)(c.y - o.y), (float)(c.z - o.z), 0.0f);
+                else
+                    ctr[slot * kK + threadIdx.x] = c;
+            }
+        };
+        double acc[T];
 #pragma unroll
-    for (int t = 0; t < T; ++t) acc[t] = 0.0;
-    if (!kSplit || first < f1) gather(first, (int)min((int64_t)kK, f1 - first), fbuf, 0);
-    cp_async_commit();
-    int sb = 0;
-    for (int64_t s0 = first; !kSplit || s0 < f1; sb ^= 1) {
-        const int n = (int)min((int64_t)kK, f1 - s0);
-        const int64_t s1 = kSplit ? s0 + step : s0 + n;
-        if (s1 < f1) gather(s1, (int)min((int64_t)kK, f1 - s1), fbuf + (size_t)(sb ^ 1) * kK * kUnits, sb ^ 1);
+        for (int t = 0; t < T; ++t) acc[t] = 0.0;
+        if (!kSplit || first < f1) gather(first, (int)min((int64_t)kK, f1 - first), fbuf, 0);
         cp_async_commit();
-        cp_async_wait_prev();
-        __syncthreads();  // stage sb resident
-        if (live) {
-            const float4* buf = fbuf + (size_t)sb * kK * kUnits;
-            if constexpr (T == 2) {
-                const float4* cs = ctrf + sb * kK;
-                float acc32[2] = {0.0f, 0.0f};
-                for (int k = 0; k < n; ++k) {
-                    const float4 c = cs[k];
-                    float rinv[2], e[2][4];
+        int sb = 0;
+        for (int64_t s0 = first; !kSplit || s0 < f1; sb ^= 1) {
+            const int n = (int)min((int64_t)kK, f1 - s0);
+            const int64_t s1 = kSplit ? s0 + step : s0 + n;
+            if (s1 < f1) gather(s1, (int)min((int64_t)kK, f1 - s1), fbuf + (size_t)(sb ^ 1) * kK * kUnits, sb ^ 1);
+            cp_async_commit();
+            cp_async_wait_prev();
+            __syncthreads();  // stage sb resident
+            if (live) {
+                const float4* buf = fbuf + (size_t)sb * kK * kUnits;
+                if constexpr (T == 2) {
+                    const float4* cs = ctrf + sb * kK;
+                    float acc32[2] = {0.0f, 0.0f};
+                    for (int k = 0; k < n; ++k) {
+                        const float4 c = cs[k];
+                        float rinv[2], e[2][4];
 #pragma unroll
-                    for (int t = 0; t < 2; ++t) {
-                        const float dx = c.x - xo[t][0], dy = c.y - xo[t][1], dz = c.z - xo[t][2];
-                        rinv[t] = rsqrt_t(dx * dx + dy * dy + dz * dz);
-                        const float s2 = rinv[t] * rinv[t];
-                        e[t][0] = dx * s2; e[t][1] = dy * s2; e[t][2] = dz * s2; e[t][3] = s2;
+                        for (int t = 0; t < 2; ++t) {
+                            const float dx = c.x - xo[t][0], dy = c.y - xo[t][1], dz = c.z - xo[t][2];
+                            rinv[t] = rsqrt_t(dx * dx + dy * dy + dz * dz);
+                            const float s2 = rinv[t] * rinv[t];
+                            e[t][0] = dx * s2; e[t][1] = dy * s2; e[t][2] = dz * s2; e[t][3] = s2;
+                        }
+                        float g[2];
+                        horner1x2<P>((const float*)(buf + (size_t)k * kUnits), e, g);
+                        acc32[0] = fmaf(rinv[0], g[0], acc32[0]);
+                        acc32[1] = fmaf(rinv[1], g[1], acc32[1]);
                     }
-                    float g[2];
-                    horner1x2<P>((const float*)(buf + (size_t)k * kUnits), e, g);
-                    acc32[0] = fmaf(rinv[0], g[0], acc32[0]);
-                    acc32[1] = fmaf(rinv[1], g[1], acc32[1]);
-                }
-                acc[0] += (double)acc32[0];
-                acc[1] += (double)acc32[1];
-            } else {
-                const double4* cs = ctr + sb * kK;
-                for (int k = 0; k < n; ++k) {
-                    const F dx = (F)(cs[k].x - x[0].x), dy = (F)(cs[k].y - x[0].y), dz = (F)(cs[k].z - x[0].z);
-                    const F rinv = rsqrt_t(dx * dx + dy * dy + dz * dz);
-                    const F s2 = rinv * rinv;
-                    const F* row = (const F*)(buf + (size_t)k * kUnits);
-                    acc[0] += (double)(rinv * horner1<P, F>(row, dx * s2, dy * s2, dz * s2, s2));
+                    acc[0] += (double)acc32[0];
+                    acc[1] += (double)acc32[1];
+                } else {
+                    const double4* cs = ctr + sb * kK;
+                    for (int k = 0; k < n; ++k) {
+                        const F dx = (F)(cs[k].x - x[0].x), dy = (F)(cs[k].y - x[0].y), dz = (F)(cs[k].z - x[0].z);
+                        const F rinv = rsqrt_t(dx * dx + dy * dy + dz * dz);
+                        const F s2 = rinv * rinv;
+                        const F* row = (const F*)(buf + (size_t)k * kUnits);
+                        acc[0] += (double)(rinv * horner1<P, F>(row, dx * s2, dy * s2, dz * s2, s2));
+                    }
                 }
             }
+            if (s1 >= f1) break;
+            __syncthreads();  // stage sb consumed before it is refilled
+            s0 = s1;
         }
-        if (s1 >= f1) break;
-        __syncthreads();  // stage sb consumed before it is refilled
-        s0 = s1;
-    }
-    if constexpr (kSplit) {  // block 0 adds the blocks' sums in rank order
-        double* red = reinterpret_cast<double*>(fbuf);
-        __syncthreads();  // the last stage is consumed
-        if (cp.rank > 0)
+        if constexpr (kSplit) {  // block 0 adds the blocks' sums in rank order
+            double* red = reinterpret_cast<double*>(fbuf);
+            __syncthreads();  // the last stage is consumed
+            if (cp.rank > 0)
 #pragma unroll
-            for (int t = 0; t < T; ++t) red[t * kNT + threadIdx.x] = acc[t];
-        cluster_barrier();
+                for (int t = 0; t < T; ++t) red[t * kNT + threadIdx.x] = acc[t];
+            cluster_barrier();
+            if (cp.rank == 0)
+                for (int r = 1; r < cp.parts; ++r)
+#pragma unroll
+                    for (int t = 0; t < T; ++t) acc[t] += cluster_load(red + t * kNT + threadIdx.x, r);
+            cluster_barrier();  // the sums are read before their space is filled again
+        }
         if (cp.rank == 0)
-            for (int r = 1; r < cp.parts; ++r)
 #pragma unroll
-                for (int t = 0; t < T; ++t) acc[t] += cluster_load(red + t * kNT + threadIdx.x, r);
-        cluster_barrier();  // the sums are read before their space is filled again
-    }
-    if (cp.rank == 0)
-#pragma unroll
-        for (int t = 0; t < T; ++t)
-            if (q + 32 * t < qe) A.V[q + 32 * t] += acc[t];
+            for (int t = 0; t < T; ++t)
+                if (q + 32 * t < qe) A.V[q + 32 * t] += acc[t];
     }
 }
 
@@ -3362,7 +3362,6 @@ static NearArgs near_args(const TreeSolver* t, double* U) {
     return N;
 }
 
-// Order P's far-field launch(es) of t on its context's stream, on the schedule tree_prepare made.
 // Blocks per batch of the far and near launches, by the batches there are for each SM (about 110 targets each).  A batch
 // is a chain of stages; with few batches the longest chains decide, and a cluster shortens them, for three cluster
 // barriers a batch.  Measured, us per evaluation with 1 / 2 / 4 blocks a batch in both launches: fixed order 8 on 15,000
@@ -3388,6 +3387,7 @@ static unsigned cluster_grid(unsigned blocks, int parts) {
     return std::max(1u, blocks / (unsigned)parts) * (unsigned)parts;
 }
 
+// Order P's far-field launch(es) of t on its context's stream, on the schedule tree_prepare made.
 static int tree_far_order(TreeSolver* t, int P, int parts) {
     lpm_ctx* ctx = t->ctx;
     FarArgs F = far_args(t, P);
